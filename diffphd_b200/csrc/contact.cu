@@ -16,16 +16,14 @@
 #include <cuda_runtime.h>
 
 #include "kernels.cuh"
+#include "launch.cuh"
+#include "ncp_common.cuh"
 
 namespace dphd {
 
 namespace {
 
-__device__ __forceinline__ double warp_sum_d(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
+__device__ __forceinline__ double warp_sum_d(double v) { return ncp_warp_sum(v); }
 
 // G_ij for i <= j, one warp per pair (prefix of matching rows from the root).
 __global__ void __launch_bounds__(256) k_delassus(int K, const int64_t* __restrict__ off, const int* __restrict__ prow,
@@ -61,77 +59,121 @@ __global__ void __launch_bounds__(256) k_delassus(int K, const int64_t* __restri
     }
 }
 
-// Block-wide exclusive scan of 0/1 flags over K candidates (one CTA), producing the ordered active list.
-__global__ void __launch_bounds__(1024) k_ncp_prepare(ContactDev c, const double* __restrict__ x, Ctrl* ctrl) {
+// Fischer-Burmeister terms of every candidate, the active flags and the ordered active list.  The candidates are
+// spread over the grid (one flag bit each, a word per warp); the block that arrives last compacts the bit words in
+// order.  Candidates outside the active set carry no friction and no contact force: their tangential multipliers are
+// cleared and their S-pass input becomes r64 (or 0).  One CTA took 15 us over 4,913 candidates and 42 us over 15,625
+// (three block barriers per 1,024 candidates in series).
+constexpr int kPrepThreads = 256;
+__global__ void __launch_bounds__(kPrepThreads) k_ncp_prepare(ContactDev c, const double* __restrict__ x,
+                                                              const double* __restrict__ r64, Ctrl* ctrl) {
+    pdl_enter();
     if (ctrl->done) return;
-    __shared__ int warp_tot[32];
-    __shared__ int base_s;
-    if (threadIdx.x == 0) base_s = 0;
-    __syncthreads();
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int b0 = 0; b0 < c.K; b0 += blockDim.x) {
-        const int k = b0 + threadIdx.x;
-        int act = 0;
-        if (k < c.K) {
-            const int node = c.cand[k];
-            const double dj = c.n[0] * x[3 * node] + c.n[1] * x[3 * node + 1] + c.n[2] * x[3 * node + 2] + c.offset;
-            const double lj = c.lam[k], rj = c.rprec[k];
-            double den = sqrt(dj * dj + rj * rj * lj * lj);
-            if (den < 1e-14) den = 1e-14;
-            const double om = 1.0 - dj / den;
-            const double E = (1.0 - rj * lj / den) * rj;
-            const double phi = dj + rj * lj - den;
-            const double Hq = dj - c.offset;
-            c.omega[k] = om;
-            c.Ediag[k] = E;
-            c.hvec[k] = -phi + om * Hq;
-            act = (lj > 0.0 || dj <= 0.0) ? 1 : 0;
+    const int k = blockIdx.x * kPrepThreads + threadIdx.x;
+    int act = 0;
+    if (k < c.K) {
+        const int node = c.cand[k];
+        const double dj = c.n[0] * x[3 * node] + c.n[1] * x[3 * node + 1] + c.n[2] * x[3 * node + 2] + c.offset;
+        const double lj = c.lam[k], rj = c.rprec[k];
+        double den = sqrt(dj * dj + rj * rj * lj * lj);
+        if (den < 1e-14) den = 1e-14;
+        const double om = 1.0 - dj / den;
+        const double E = (1.0 - rj * lj / den) * rj;
+        const double phi = dj + rj * lj - den;
+        const double Hq = dj - c.offset;
+        c.omega[k] = om;
+        c.Ediag[k] = E;
+        c.hvec[k] = -phi + om * Hq;
+        act = (lj > 0.0 || dj <= 0.0) ? 1 : 0;
+        if (!act) {
+            c.lt1[k] = c.lt2[k] = 0.0;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) c.vc[3 * (size_t)k + d] = r64 ? r64[3 * node + d] : 0.0;
         }
-        // scan
-        const unsigned bal = __ballot_sync(0xffffffffu, act);
-        const int pre = __popc(bal & ((1u << lane) - 1u));
-        if (lane == 0) warp_tot[wid] = __popc(bal);
-        __syncthreads();
-        int woff = 0;
-        for (int w = 0; w < wid; ++w) woff += warp_tot[w];
-        if (act) c.act[base_s + woff + pre] = k;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int t = 0;
-            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += warp_tot[w];
-            base_s += t;
+    }
+    const unsigned bal = __ballot_sync(0xffffffffu, act);
+    if (lane == 0 && k < c.K) c.act_mask[k >> 5] = bal;
+    // last block: ordered compaction of the bit words
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(reinterpret_cast<unsigned int*>(c.ncp_flags) + 4, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __shared__ int warp_tot[kPrepThreads / 32];
+    const int nw = (c.K + 31) >> 5;
+    int base = 0;
+    for (int w0 = 0; w0 < nw; w0 += kPrepThreads) {
+        const int w = w0 + threadIdx.x;
+        unsigned bits = w < nw ? __ldcg(c.act_mask + w) : 0u;
+        const int cnt = __popc(bits);
+        int pre = cnt;  // inclusive scan over the warp
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, pre, o);
+            if (lane >= o) pre += t;
         }
+        if (lane == 31) warp_tot[wid] = pre;
+        __syncthreads();
+        int woff = 0, tot = 0;
+#pragma unroll
+        for (int v = 0; v < kPrepThreads / 32; ++v) {
+            if (v < wid) woff += warp_tot[v];
+            tot += warp_tot[v];
+        }
+        int o = base + woff + pre - cnt;
+        while (bits) {
+            c.act[o++] = 32 * w + __ffs(bits) - 1;
+            bits &= bits - 1;
+        }
+        base += tot;
         __syncthreads();
     }
-    if (threadIdx.x == 0) c.kact[0] = base_s;
+    if (threadIdx.x == 0) {
+        c.kact[0] = base;
+        c.ncp_flags[4] = 0;
+    }
 }
 
-// A^-1 b at active candidate nodes: dot of the node's S column path with y = S b (3 right-hand sides).
-template <typename T>
-__global__ void __launch_bounds__(256) k_ncp_ainvb(ContactDev c, const T* __restrict__ y, int npad,
-                                                   const double* __restrict__ x_base, const Ctrl* ctrl) {
+// A^-1 b at active candidate nodes: dot of the node's S column path with y = S b (3 right-hand sides), one CTA per
+// active candidate (a path of a thousand rows is a chain of dependent row and y loads: one warp took 16 us for it).
+constexpr int kDotThreads = 256;
+__global__ void __launch_bounds__(kDotThreads) k_ncp_ainvb(ContactDev c, const double* __restrict__ y, int npad,
+                                                           const double* __restrict__ x_base, const Ctrl* ctrl) {
+    pdl_enter();
     if (ctrl->done) return;
-    const int a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (a >= c.kact[0]) return;
-    const int k = c.act[a];
-    const int64_t o = c.off[k];
-    const int L = (int)(c.off[k + 1] - o);
-    double s0 = 0, s1 = 0, s2 = 0;
-    for (int d = lane; d < L; d += 32) {
-        const int r = c.prow[o + d];
-        const double v = c.pval[o + d];
-        s0 += v * (double)y[r];
-        s1 += v * (double)y[npad + r];
-        s2 += v * (double)y[2 * (size_t)npad + r];
-    }
-    s0 = warp_sum_d(s0);
-    s1 = warp_sum_d(s1);
-    s2 = warp_sum_d(s2);
-    if (lane == 0) {
-        const int node = c.cand[k];
-        c.ainvb[3 * a] = s0 + (x_base ? x_base[3 * node] : 0.0);
-        c.ainvb[3 * a + 1] = s1 + (x_base ? x_base[3 * node + 1] : 0.0);
-        c.ainvb[3 * a + 2] = s2 + (x_base ? x_base[3 * node + 2] : 0.0);
+    __shared__ double sh[3][kDotThreads / 32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int ka = c.kact[0];
+    for (int a = blockIdx.x; a < ka; a += gridDim.x) {
+        const int k = c.act[a];
+        const int64_t o = c.off[k];
+        const int L = (int)(c.off[k + 1] - o);
+        double s0 = 0, s1 = 0, s2 = 0;
+        for (int d = threadIdx.x; d < L; d += kDotThreads) {
+            const int r = c.prow[o + d];
+            const double v = c.pval[o + d];
+            s0 += v * y[r];
+            s1 += v * y[npad + r];
+            s2 += v * y[2 * (size_t)npad + r];
+        }
+        s0 = warp_sum_d(s0);
+        s1 = warp_sum_d(s1);
+        s2 = warp_sum_d(s2);
+        if (lane == 0) {
+            sh[0][wid] = s0;
+            sh[1][wid] = s1;
+            sh[2][wid] = s2;
+        }
+        __syncthreads();
+        if (threadIdx.x < 3) {
+            double s = 0.0;
+#pragma unroll
+            for (int w = 0; w < kDotThreads / 32; ++w) s += sh[threadIdx.x][w];
+            c.ainvb[3 * a + threadIdx.x] = s + (x_base ? x_base[3 * c.cand[k] + threadIdx.x] : 0.0);
+        }
+        __syncthreads();
     }
 }
 
@@ -214,32 +256,18 @@ __device__ void ncp_tile_cholesky(double* sD) {
     }
 }
 
-template <typename T>
 __global__ void __launch_bounds__(kNcpThreads, 1)
-k_ncp_block_solve(ContactDev c, const double* __restrict__ q0, const int* __restrict__ iperm, T* __restrict__ vcon,
-                  int npad, const double* __restrict__ r64, Ctrl* ctrl) {
+k_ncp_block_solve(ContactDev c, const double* __restrict__ q0, const double* __restrict__ r64, Ctrl* ctrl) {
     extern __shared__ double smem[];
     double* sA = smem;                           // 64 x kNcpLd: diagonal block / k-major panel i
     double* sB = smem + kNcpTile * kNcpLd;       // 64 x kNcpLd: panel tile / k-major panel j
     double* sy = smem + 2 * kNcpTile * kNcpLd;   // 64: the block's right-hand side / solution
     if (ctrl->done) return;  // every CTA reads the same value: no CTA reaches a barrier the others skip
-    const int K = c.K, ka = c.kact[0];
+    const int ka = c.kact[0];
     const int tid = threadIdx.x, nt = blockDim.x, G = gridDim.x, bid = blockIdx.x;
     const int gt = bid * nt + tid, nthr = G * nt;
     const int lane = tid & 31, gw = gt >> 5, nwarps = nthr >> 5;
-    const double n0 = c.n[0], n1 = c.n[1], n2 = c.n[2];
-    // clear the previous contact right-hand side at every candidate node
-    for (int k = gt; k < K; k += nthr) {
-        const int node = c.cand[k], j = iperm[node];
-        vcon[j] = r64 ? (T)r64[3 * node] : T(0);
-        vcon[npad + j] = r64 ? (T)r64[3 * node + 1] : T(0);
-        vcon[2 * (size_t)npad + j] = r64 ? (T)r64[3 * node + 2] : T(0);
-        for (int d = 0; d < 3; ++d) c.vc[3 * (size_t)k + d] = r64 ? r64[3 * node + d] : 0.0;
-    }
-    if (ka == 0) {
-        for (int k = gt; k < K; k += nthr) c.lt1[k] = c.lt2[k] = 0.0;
-        return;
-    }
+    if (ka == 0) return;
     const int nb = (ka + kNcpTile - 1) / kNcpTile, ld = nb * kNcpTile;
     double* M = c.Mwork;  // ld x ld, row-major, lower triangle used
     double* rhs = c.rhs;  // ld
@@ -251,29 +279,10 @@ k_ncp_block_solve(ContactDev c, const double* __restrict__ q0, const int* __rest
             if (lane == 0) rhs[a] = 0.0;
             continue;
         }
-        const int k = c.act[a];
-        const double om = c.omega[k];
-        const double* Gk = c.G + (size_t)k * K;
-        double g0 = 0.0, g1 = 0.0, g2 = 0.0;
-        for (int b = lane; b < ka; b += 32) {
-            const int kb = c.act[b];
-            const double Gab = Gk[kb];
-            const double fn = c.omega[kb] * c.lam[kb];
-            const double f1 = c.lt1[kb], f2 = c.lt2[kb];
-            g0 += Gab * (fn * n0 + f1 * c.t1[0] + f2 * c.t2[0]);
-            g1 += Gab * (fn * n1 + f1 * c.t1[1] + f2 * c.t2[1]);
-            g2 += Gab * (fn * n2 + f1 * c.t1[2] + f2 * c.t2[2]);
-            if (b <= a) Ma[b] = om * Gab * c.omega[kb] + (a == b ? c.Ediag[k] : 0.0);
-        }
-        g0 = warp_sum_d(g0);
-        g1 = warp_sum_d(g1);
-        g2 = warp_sum_d(g2);
-        if (lane == 0) {
-            g0 += c.ainvb[3 * a];
-            g1 += c.ainvb[3 * a + 1];
-            g2 += c.ainvb[3 * a + 2];
-            rhs[a] = c.hvec[k] - om * (n0 * g0 + n1 * g1 + n2 * g2);
-        }
+        const double h = ncp_row(c, a, ka, lane, [&](int b, double m) {
+            if (b <= a) Ma[b] = m;
+        });
+        if (lane == 0) rhs[a] = h;
     }
     if (!ncp_grid_sync(c.bar, ctrl)) return;
     // ---- B: blocked factorisation with the forward substitution folded in ----
@@ -442,71 +451,10 @@ k_ncp_block_solve(ContactDev c, const double* __restrict__ q0, const int* __rest
         }
         if (!ncp_grid_sync(c.bar, ctrl)) return;
     }
-    // ---- D: multipliers, Coulomb cone (forward_gpu.cpp:1255-1302), contact right-hand side ----
-    for (int a = gt; a < ka; a += nthr) {
-        const int k = c.act[a];
-        double l = c.lam[k] + c.xsol[a];
-        l = l < 0.0 ? 0.0 : (l > 1e8 ? 1e8 : l);
-        c.lam[k] = l;
-    }
-    for (int k = gt; k < K; k += nthr) c.lt1[k] = c.lt2[k] = 0.0;  // non-active candidates carry no friction
+    // ---- D: multipliers, Coulomb cone, contact right-hand side ----
+    for (int a = gt; a < ka; a += nthr) ncp_clamp_row(c, c.act[a], c.xsol[a]);
     if (!ncp_grid_sync(c.bar, ctrl)) return;
-    for (int a = gw; a < ka; a += nwarps) {
-        const int k = c.act[a];
-        double t1v = 0.0, t2v = 0.0;
-        if (c.mu > 0.0 && c.lam[k] > 0.0) {
-            const double* Gk = c.G + (size_t)k * K;
-            double f = 0.0;
-            for (int b = lane; b < ka; b += 32) {
-                const int kb = c.act[b];
-                f += c.omega[kb] * c.lam[kb] * Gk[kb];
-            }
-            f = warp_sum_d(f);
-            const int node = c.cand[k];
-            const double qn0 = c.ainvb[3 * a] + f * n0, qn1 = c.ainvb[3 * a + 1] + f * n1,
-                         qn2 = c.ainvb[3 * a + 2] + f * n2;
-            const double s0 = qn0 - q0[3 * node], s1 = qn1 - q0[3 * node + 1], s2 = qn2 - q0[3 * node + 2];
-            const double sn = s0 * n0 + s1 * n1 + s2 * n2;
-            const double u0 = s0 - sn * n0, u1 = s1 - sn * n1, u2 = s2 - sn * n2;
-            const double ut1 = u0 * c.t1[0] + u1 * c.t1[1] + u2 * c.t1[2];
-            const double ut2 = u0 * c.t2[0] + u1 * c.t2[1] + u2 * c.t2[2];
-            const double Gkk = Gk[k];
-            double st1 = 0.0, st2 = 0.0;
-            if (fabs(Gkk * Gkk) > 1e-20) {
-                st1 = -ut1 / Gkk;
-                st2 = -ut2 / Gkk;
-            }
-            const double cone = c.mu * c.lam[k];
-            if (sqrt(st1 * st1 + st2 * st2) <= cone + 1e-14) {
-                t1v = st1;
-                t2v = st2;
-            } else {
-                const double um = sqrt(ut1 * ut1 + ut2 * ut2);
-                if (um > 1e-14) {
-                    t1v = -cone * ut1 / um;
-                    t2v = -cone * ut2 / um;
-                }
-            }
-        }
-        if (lane == 0) {
-            c.lt1[k] = t1v;
-            c.lt2[k] = t2v;
-            // contact right-hand side J^T f at the node (omega from this iteration times the new lambda)
-            const double fn = c.omega[k] * c.lam[k];
-            const int node = c.cand[k], j = iperm[node];
-            const double r0 = r64 ? r64[3 * node] : 0.0, r1 = r64 ? r64[3 * node + 1] : 0.0,
-                         r2 = r64 ? r64[3 * node + 2] : 0.0;
-            const double w0 = r0 + fn * n0 + t1v * c.t1[0] + t2v * c.t2[0];
-            const double w1 = r1 + fn * n1 + t1v * c.t1[1] + t2v * c.t2[1];
-            const double w2 = r2 + fn * n2 + t1v * c.t1[2] + t2v * c.t2[2];
-            vcon[j] = (T)w0;
-            vcon[npad + j] = (T)w1;
-            vcon[2 * (size_t)npad + j] = (T)w2;
-            c.vc[3 * (size_t)k] = w0;
-            c.vc[3 * (size_t)k + 1] = w1;
-            c.vc[3 * (size_t)k + 2] = w2;
-        }
-    }
+    for (int a = gw; a < ka; a += nwarps) ncp_finish_row(c, a, ka, lane, q0, r64);
 }
 
 // Restitution (forward_gpu.cpp:1483-1531), planar boundary.
@@ -546,24 +494,18 @@ void launch_delassus(int K, const int64_t* off, const int* prow, const double* p
     if (npairs > 0) k_delassus<<<(unsigned)blocks, 256, 0, st>>>(K, off, prow, pval, G);
 }
 
-template <typename T>
-void launch_ncp_iteration(const ContactDev& c, const double* x, const T* y, int npad, const double* x_base,
-                          const double* q0, const int* iperm, T* vcon, const double* r64, Ctrl* ctrl,
-                          cudaStream_t st) {
-    k_ncp_prepare<<<1, 1024, 0, st>>>(c, x, ctrl);
-    k_ncp_ainvb<T><<<(c.K * 32 + 255) / 256, 256, 0, st>>>(c, y, npad, x_base, ctrl);
+void launch_ncp_iteration(const ContactDev& c, const double* x, const double* y, int npad, const double* x_base,
+                          const double* q0, const double* r64, Ctrl* ctrl, cudaStream_t st) {
+    launch_k(k_ncp_prepare, (c.K + kPrepThreads - 1) / kPrepThreads, kPrepThreads, 0, st, c, x, r64, ctrl);
+    launch_k(k_ncp_ainvb, c.K < 4 * ncp_grid() ? c.K : 4 * ncp_grid(), kDotThreads, 0, st, c, y, npad, x_base,
+             (const Ctrl*)ctrl);
     if (c.cached) {
-        launch_ncp_cached_solve<T>(c, q0, iperm, vcon, npad, r64, ctrl, st);
+        launch_ncp_cached_solve(c, q0, r64, ctrl, st);
         return;
     }
     // one cooperative grid of one CTA per SM (the barrier needs every CTA resident)
     const size_t smem = (size_t)(2 * kNcpTile * kNcpLd + kNcpTile) * sizeof(double);
-    static bool attr_set[2] = {false, false};
-    void (*kern)(ContactDev, const double*, const int*, T*, int, const double*, Ctrl*) = k_ncp_block_solve<T>;
-    if (!attr_set[sizeof(T) == 8]) {
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        attr_set[sizeof(T) == 8] = true;
-    }
+    cudaFuncSetAttribute(k_ncp_block_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ncp_grid());
     cfg.blockDim = dim3(kNcpThreads);
@@ -574,30 +516,50 @@ void launch_ncp_iteration(const ContactDev& c, const double* x, const T* y, int 
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kern, c, q0, iperm, vcon, npad, r64, ctrl);
+    cudaLaunchKernelEx(&cfg, k_ncp_block_solve, c, q0, r64, ctrl);
 }
-template void launch_ncp_iteration<double>(const ContactDev&, const double*, const double*, int, const double*,
-                                           const double*, const int*, double*, const double*, Ctrl*, cudaStream_t);
-template void launch_ncp_iteration<float>(const ContactDev&, const double*, const float*, int, const double*,
-                                          const double*, const int*, float*, const double*, Ctrl*, cudaStream_t);
 
 namespace {
+// One warp per row of U.  v supported on few candidates (`list`): a lane per candidate looks its path up at the row's
+// depth -- the row lies on the path of candidate k exactly when the path's entry at that depth is the row -- so a row
+// costs `count` look-ups instead of a pass over every candidate below it.  With every node of a block a candidate and
+// 3 to 9 of them in contact the row lists hold all of S (24^3: 249 us per apply; the look-ups 6 us).  A look-up is a
+// 32-byte sector where a list entry is 12 streamed bytes and a 24-byte gather, hence the factor in the rule.
+constexpr int kPathLookupCost = 4;
 template <typename TI, typename TO>
 __global__ void __launch_bounds__(256) k_path_apply(ContactDev c, const double* __restrict__ vsrc, int from_nodes,
+                                                    const int* __restrict__ list, const int* __restrict__ count,
                                                     const TI* yin, TO* yout, int npad, const Ctrl* ctrl) {
+    pdl_enter();
     if (ctrl->done) return;
     const int u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (u >= c.nU) return;
     const int row = c.tp_row[u];
-    const int64_t e0 = c.tp_ptr[u], e1 = c.tp_ptr[u + 1];
+    const int cnt = list ? *count : 0;
     double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-    for (int64_t e = e0 + lane; e < e1; e += 32) {
-        const int k = c.tp_k[e];
-        const double v = c.tp_val[e];
-        const double* src = vsrc + 3 * (size_t)(from_nodes ? c.cand[k] : k);
-        s0 += v * src[0];
-        s1 += v * src[1];
-        s2 += v * src[2];
+    if (list && (long long)cnt * c.nU * kPathLookupCost <= c.tp_entries) {
+        const int depth = c.tp_depth[u];
+        for (int a = lane; a < cnt; a += 32) {
+            const int k = list[a];
+            const int64_t o = c.off[k] + depth;
+            if (o < c.off[k + 1] && c.prow[o] == row) {
+                const double v = c.pval[o];
+                const double* src = vsrc + 3 * (size_t)(from_nodes ? c.cand[k] : k);
+                s0 += v * src[0];
+                s1 += v * src[1];
+                s2 += v * src[2];
+            }
+        }
+    } else {
+        const int64_t e0 = c.tp_ptr[u], e1 = c.tp_ptr[u + 1];
+        for (int64_t e = e0 + lane; e < e1; e += 32) {
+            const int k = c.tp_k[e];
+            const double v = c.tp_val[e];
+            const double* src = vsrc + 3 * (size_t)(from_nodes ? c.cand[k] : k);
+            s0 += v * src[0];
+            s1 += v * src[1];
+            s2 += v * src[2];
+        }
     }
     s0 = warp_sum_d(s0);
     s1 = warp_sum_d(s1);
@@ -612,6 +574,7 @@ __global__ void __launch_bounds__(256) k_path_apply(ContactDev c, const double* 
 
 __global__ void k_cand_zero(ContactDev c, const int* __restrict__ iperm, float* __restrict__ v, int npad,
                             const Ctrl* ctrl) {
+    pdl_enter();
     if (ctrl->done) return;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= c.K) return;
@@ -630,20 +593,22 @@ __global__ void k_path_gather_vals(long long E, const int64_t* __restrict__ src_
 
 template <typename TI, typename TO>
 void launch_path_apply(const ContactDev& c, const double* v_src, int from_nodes, const TI* y_in, TO* y_out, int npad,
-                       const Ctrl* ctrl, cudaStream_t st) {
+                       const Ctrl* ctrl, cudaStream_t st, const int* list, const int* count) {
     if (c.nU <= 0) return;
-    k_path_apply<TI, TO><<<(unsigned)(((long long)c.nU * 32 + 255) / 256), 256, 0, st>>>(c, v_src, from_nodes, y_in,
-                                                                                        y_out, npad, ctrl);
+    launch_k(k_path_apply<TI, TO>, (unsigned)(((long long)c.nU * 32 + 255) / 256), 256, 0, st, c, v_src, from_nodes,
+             list, count, y_in, y_out, npad, ctrl);
 }
 template void launch_path_apply<double, double>(const ContactDev&, const double*, int, const double*, double*, int,
-                                                const Ctrl*, cudaStream_t);
+    const Ctrl*, cudaStream_t, const int*, const int*);
+template void launch_path_apply<double, float>(const ContactDev&, const double*, int, const double*, float*, int,
+    const Ctrl*, cudaStream_t, const int*, const int*);
 template void launch_path_apply<float, double>(const ContactDev&, const double*, int, const float*, double*, int,
-                                               const Ctrl*, cudaStream_t);
+    const Ctrl*, cudaStream_t, const int*, const int*);
 template void launch_path_apply<float, float>(const ContactDev&, const double*, int, const float*, float*, int,
-                                              const Ctrl*, cudaStream_t);
+    const Ctrl*, cudaStream_t, const int*, const int*);
 
 void launch_cand_zero(const ContactDev& c, const int* iperm, float* v, int npad, const Ctrl* ctrl, cudaStream_t st) {
-    if (c.K > 0) k_cand_zero<<<(c.K + 255) / 256, 256, 0, st>>>(c, iperm, v, npad, ctrl);
+    if (c.K > 0) launch_k(k_cand_zero, (c.K + 255) / 256, 256, 0, st, c, iperm, v, npad, ctrl);
 }
 
 void launch_path_gather_vals(long long E, const int64_t* src_e, const double* pval, double* tp_val, cudaStream_t st) {

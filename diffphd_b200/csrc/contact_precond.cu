@@ -23,33 +23,53 @@ __device__ __forceinline__ double wsum(double v) {
     return v;
 }
 
+// u_b = d_b . (A^-1 r) at the constrained nodes: one CTA per node over its S column path (one warp took 27 us for three
+// paths of a thousand rows: a chain of dependent loads).
+constexpr int kDotThreads = 256;
 template <typename T>
-__global__ void __launch_bounds__(256) k_wbp_jdot(const int* __restrict__ count, const int* __restrict__ wcand,
-                                                  const int* __restrict__ wpos, ContactDev c, const T* __restrict__ y,
-                                                  int npad, WbpDirs dirs, int cap, double* __restrict__ u,
-                                                  const Ctrl* ctrl) {
+__global__ void __launch_bounds__(kDotThreads) k_wbp_jdot(const int* __restrict__ count, const int* __restrict__ wcand,
+                                                          const int* __restrict__ wpos, ContactDev c,
+                                                          const T* __restrict__ y, int npad, WbpDirs dirs, int cap,
+                                                          double* __restrict__ u, const Ctrl* ctrl) {
     if (ctrl->done) return;
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (i >= *count) return;
-    const int k = wcand[i];
-    const int64_t o = c.off[k];
-    const int L = (int)(c.off[k + 1] - o);
-    double s0 = 0, s1 = 0, s2 = 0;
-    for (int d = lane; d < L; d += 32) {
-        const int r = c.prow[o + d];
-        const double v = c.pval[o + d];
-        s0 += v * (double)y[r];
-        s1 += v * (double)y[npad + r];
-        s2 += v * (double)y[2 * (size_t)npad + r];
-    }
-    s0 = wsum(s0);
-    s1 = wsum(s1);
-    s2 = wsum(s2);
-    if (lane == 0)
-        for (int b = 0; b < 3; ++b) {
-            const int pos = wpos[3 * i + b];
-            if (pos >= 0) u[b * cap + pos] = dirs.d[b][0] * s0 + dirs.d[b][1] * s1 + dirs.d[b][2] * s2;
+    __shared__ double sh[3][kDotThreads / 32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int n = *count;
+    for (int i = blockIdx.x; i < n; i += gridDim.x) {
+        const int k = wcand[i];
+        const int64_t o = c.off[k];
+        const int L = (int)(c.off[k + 1] - o);
+        double s0 = 0, s1 = 0, s2 = 0;
+        for (int d = threadIdx.x; d < L; d += kDotThreads) {
+            const int r = c.prow[o + d];
+            const double v = c.pval[o + d];
+            s0 += v * (double)y[r];
+            s1 += v * (double)y[npad + r];
+            s2 += v * (double)y[2 * (size_t)npad + r];
         }
+        s0 = wsum(s0);
+        s1 = wsum(s1);
+        s2 = wsum(s2);
+        if (lane == 0) {
+            sh[0][wid] = s0;
+            sh[1][wid] = s1;
+            sh[2][wid] = s2;
+        }
+        __syncthreads();
+        if (threadIdx.x < 3) {
+            const int pos = wpos[3 * i + threadIdx.x];
+            if (pos >= 0) {
+                double t[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+                for (int w = 0; w < kDotThreads / 32; ++w)
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) t[d] += sh[d][w];
+                const double* db = dirs.d[threadIdx.x];
+                u[threadIdx.x * cap + pos] = db[0] * t[0] + db[1] * t[1] + db[2] * t[2];
+            }
+        }
+        __syncthreads();
+    }
 }
 
 // w_b = X_b u_b (X_b lower triangular at X + b * ld * ld, leading dimension ld); one warp per row.
@@ -145,7 +165,7 @@ void launch_wbp_precond_parts(int stage, int cap, const int* count, const int* w
     if (cap <= 0) return;
     if (stage == 0) {  // u = J A^-1 r, lam = (J A^-1 J^T)^-1 u (X: three blocks, then their three transposes)
         const double* Xt = X + (size_t)3 * ld * ld;
-        k_wbp_jdot<T><<<(cap * 32 + 255) / 256, 256, 0, st>>>(count, wcand, wpos, c, y, npad, dirs, cap, u, ctrl);
+        k_wbp_jdot<T><<<cap < 4 * ncp_grid() ? cap : 4 * ncp_grid(), kDotThreads, 0, st>>>(count, wcand, wpos, c, y, npad, dirs, cap, u, ctrl);
         k_wbp_trmv<<<(unsigned)(((long long)3 * cap * 32 + 255) / 256), 256, 0, st>>>(nb, X, ld, u, w, cap, ctrl);
         k_wbp_trmvt<<<(unsigned)(((long long)3 * cap * 32 + 255) / 256), 256, 0, st>>>(nb, Xt, ld, w, lam, cap, ctrl);
     } else {  // the S-pass input -J^T lam, per candidate

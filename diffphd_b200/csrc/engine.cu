@@ -644,8 +644,6 @@ void Engine::build_device(int threads) {
         Acsr_.v = d_A_v.as<double>();
     }
     d_q0.alloc(ld * sizeof(double));
-    d_vcon.alloc((size_t)npad_ * 3 * sizeof(double));
-    CUDA_OK(cudaMemset(d_vcon.p, 0, d_vcon.bytes));
     d_r64.alloc((size_t)n3 * sizeof(double));
     build_contact(built_dt_);
     drop_graphs();
@@ -703,12 +701,15 @@ void Engine::build_contact(double dt) {
         const int64_t E = P.off[K];
         std::vector<int> cnt(M.n, 0);
         for (int64_t e = 0; e < E; ++e) cnt[P.row[e]]++;
-        std::vector<int> urow;
+        std::vector<int> urow, depth(M.n, 0), udepth;
+        for (int k = 0; k < K; ++k)
+            for (int64_t e = P.off[k]; e < P.off[k + 1]; ++e) depth[P.row[e]] = (int)(e - P.off[k]);
         std::vector<int64_t> uptr(1, 0), rpos(M.n, -1);
         for (int r = 0; r < M.n; ++r)
             if (cnt[r]) {
                 rpos[r] = uptr.back();
                 urow.push_back(r);
+                udepth.push_back(depth[r]);
                 uptr.push_back(uptr.back() + cnt[r]);
             }
         std::vector<int> tk(E);
@@ -720,6 +721,7 @@ void Engine::build_contact(double dt) {
                 te[q] = e;
             }
         dc_tprow.upload(urow);
+        dc_tpdepth.upload(udepth);
         dc_tpptr.upload(uptr);
         dc_tpk.upload(tk);
         DeviceBuffer src;
@@ -731,6 +733,12 @@ void Engine::build_contact(double dt) {
         path_entries_ = (long long)E;
         path_max_depth_ = P.max_depth;
         c.tp_row = dc_tprow.as<int>();
+        c.tp_depth = dc_tpdepth.as<int>();
+        c.tp_entries = (long long)E;
+        // mixed precision: the FP32 S pass with two path products reads 4 bytes a value of S and about 12 a path
+        // entry each, an FP64 S pass 8 bytes a value (24^3, every node a candidate: 337 + 249 us of path products
+        // against 45 us; 64^3 with its bottom face: 39 M entries against 2.5 G values)
+        paths_hold_s_ = 24 * (double)E > 4 * (double)s_padded_values();
         c.tp_ptr = dc_tpptr.as<int64_t>();
         c.tp_k = dc_tpk.as<int>();
         c.tp_val = dc_tpval.as<double>();
@@ -766,7 +774,8 @@ void Engine::build_contact(double dt) {
     dc_refpos.alloc((size_t)K * sizeof(int));
     CUDA_OK(cudaMemset(dc_refpos.p, 0xff, dc_refpos.bytes));  // -1: no candidate is in a cached list yet
     dc_refinv.alloc(kcap * sizeof(int));
-    dc_flags.alloc(4 * sizeof(int));
+    dc_flags.alloc(8 * sizeof(int));
+    dc_mask.alloc((size_t)((K + 31) / 32) * sizeof(unsigned int));
     CUDA_OK(cudaMemset(dc_flags.p, 0, dc_flags.bytes));
     dc_stats.alloc(4 * sizeof(unsigned long long));
     CUDA_OK(cudaMemset(dc_stats.p, 0, dc_stats.bytes));
@@ -804,6 +813,7 @@ void Engine::build_contact(double dt) {
     c.ref_pos = dc_refpos.as<int>();
     c.ref_inv = dc_refinv.as<int>();
     c.ncp_flags = dc_flags.as<int>();
+    c.act_mask = dc_mask.as<unsigned int>();
     c.ncp_stats = dc_stats.as<unsigned long long>();
 }
 
@@ -867,24 +877,38 @@ void Engine::enqueue_contact_iteration(cudaStream_t st, bool f32) {
             launch_elem_fwd<double>(M.m, M.k, M.s, dE.as<int>(), d_x.as<double>(), d_qb.as<double>(),
                                     d_elem_dir.as<unsigned char>(), dgrad.as<double>(), M.hex, M.vol / M.s, ep,
                                     d_elem_out64.as<double>(), c, st);
-        launch_gather_fwd<float>(n, d_node_ptr.as<int>(), d_node_inc.as<int>(), d_elem_out64.as<double>(),
-                                 d_qt.as<double>(), inv_h2m, d_fixed_node.as<unsigned char>(), d_iperm.as<int>(),
-                                 d_vperm32.as<float>(), npad_, d_prev_pd.as<double>(), d_part_gate.as<double>(),
-                                 gather_blocks_, Acsr_, d_x.as<double>(), 1, c, st, d_r64.as<double>());
-        // One S pass on the residual away from the candidates (small near the fixed point), the candidates' part
-        // by their S column paths in FP64: r carries -J^T f there, so its FP32 image would put rounding noise
-        // into the contact gaps, and after the NCP step the S input there becomes r + J^T f (small again).
-        launch_cand_zero(contact_, d_iperm.as<int>(), d_vperm32.as<float>(), npad_, c, st);
-        launch_s_only<float>(plan32_, d_vperm32.as<float>(), d_y32.as<float>(), c, st);  // y = S r_nc
-        // S r at the rows of U, for A^-1 b = x + S^T-path(S r) at the candidates
-        launch_path_apply<float, double>(contact_, d_r64.as<double>(), 1, d_y32.as<float>(), d_y64.as<double>(), npad_,
-                                         c, st);
-        launch_ncp_iteration<double>(contact_, d_x.as<double>(), d_y64.as<double>(), npad_, d_x.as<double>(),
-                                     d_q0.as<double>(), d_iperm.as<int>(), d_vcon.as<double>(), d_r64.as<double>(),
-                                     c, st);
-        // y = S (r + J^T f): the candidates' inputs r + J^T f (FP64, from the NCP step) by their paths
-        launch_path_apply<float, float>(contact_, contact_.vc, 0, d_y32.as<float>(), d_y32.as<float>(), npad_, c,
-                                        st);
+        if (paths_hold_s_) {
+            // The candidates' column paths hold most of S (every node a candidate): the two path products below
+            // would read more bytes than S itself, so S r is one FP64 pass, and only J^T f at the active candidates
+            // goes through their paths.
+            launch_gather_fwd<double>(n, d_node_ptr.as<int>(), d_node_inc.as<int>(), d_elem_out64.as<double>(),
+                                      d_qt.as<double>(), inv_h2m, d_fixed_node.as<unsigned char>(), d_iperm.as<int>(),
+                                      d_vperm64.as<double>(), npad_, d_prev_pd.as<double>(), d_part_gate.as<double>(),
+                                      gather_blocks_, Acsr_, d_x.as<double>(), 1, c, st);
+            launch_s_only<double>(plan64_, d_vperm64.as<double>(), d_y64.as<double>(), c, st, d_y32.as<float>());
+            launch_ncp_iteration(contact_, d_x.as<double>(), d_y64.as<double>(), npad_, d_x.as<double>(),
+                                 d_q0.as<double>(), nullptr, c, st);
+            launch_path_apply<double, float>(contact_, contact_.vc, 0, d_y64.as<double>(), d_y32.as<float>(), npad_,
+                                             c, st, contact_.act, contact_.kact);
+        } else {
+            launch_gather_fwd<float>(n, d_node_ptr.as<int>(), d_node_inc.as<int>(), d_elem_out64.as<double>(),
+                                     d_qt.as<double>(), inv_h2m, d_fixed_node.as<unsigned char>(), d_iperm.as<int>(),
+                                     d_vperm32.as<float>(), npad_, d_prev_pd.as<double>(), d_part_gate.as<double>(),
+                                     gather_blocks_, Acsr_, d_x.as<double>(), 1, c, st, d_r64.as<double>());
+            // One S pass on the residual away from the candidates (small near the fixed point), the candidates' part
+            // by their S column paths in FP64: r carries -J^T f there, so its FP32 image would put rounding noise
+            // into the contact gaps, and after the NCP step the S input there becomes r + J^T f (small again).
+            launch_cand_zero(contact_, d_iperm.as<int>(), d_vperm32.as<float>(), npad_, c, st);
+            launch_s_only<float>(plan32_, d_vperm32.as<float>(), d_y32.as<float>(), c, st);  // y = S r_nc
+            // S r at the rows of U, for A^-1 b = x + S^T-path(S r) at the candidates
+            launch_path_apply<float, double>(contact_, d_r64.as<double>(), 1, d_y32.as<float>(), d_y64.as<double>(),
+                                             npad_, c, st);
+            launch_ncp_iteration(contact_, d_x.as<double>(), d_y64.as<double>(), npad_, d_x.as<double>(),
+                                 d_q0.as<double>(), d_r64.as<double>(), c, st);
+            // y = S (r + J^T f): the candidates' inputs r + J^T f (FP64, from the NCP step) by their paths
+            launch_path_apply<float, float>(contact_, contact_.vc, 0, d_y32.as<float>(), d_y32.as<float>(), npad_, c,
+                                            st);
+        }
         SpmvPlan<float> ref = plan32_;
         ref.x_base = d_x.as<double>();
         launch_st_only<float>(ref, d_y32.as<float>(), d_xraw.as<double>(), c, st);
@@ -912,10 +936,11 @@ void Engine::enqueue_contact_iteration64(cudaStream_t st) {
                               d_vperm64.as<double>(), npad_, d_prev_pd.as<double>(), d_part_gate.as<double>(),
                               gather_blocks_, NodeCsr(), nullptr, 0, c, st);
     launch_s_only<double>(plan64_, d_vperm64.as<double>(), d_y64.as<double>(), c, st);
-    launch_ncp_iteration<double>(contact_, d_x.as<double>(), d_y64.as<double>(), npad_, nullptr,
-                                 d_q0.as<double>(), d_iperm.as<int>(), d_vcon.as<double>(), nullptr, c, st);
-    // y += S J^T f by the candidates' S column paths (J^T f lives on the candidates only)
-    launch_path_apply<double, double>(contact_, contact_.vc, 0, d_y64.as<double>(), d_y64.as<double>(), npad_, c, st);
+    launch_ncp_iteration(contact_, d_x.as<double>(), d_y64.as<double>(), npad_, nullptr, d_q0.as<double>(), nullptr, c,
+                         st);
+    // y += S J^T f by the candidates' S column paths (J^T f lives on the active candidates only)
+    launch_path_apply<double, double>(contact_, contact_.vc, 0, d_y64.as<double>(), d_y64.as<double>(), npad_, c, st,
+                                      contact_.act, contact_.kact);
     launch_st_only<double>(plan64_, d_y64.as<double>(), d_xraw.as<double>(), c, st);
 }
 
@@ -1023,7 +1048,7 @@ void Engine::enqueue_contact_precond(bool f32, bool woodbury, cudaStream_t st) {
                                             d_wbp_lam.as<double>(), d_wbp_vk.as<double>(), c, st);
         // y -= S J^T lam by the constrained candidates' S column paths (FP64 sums)
         launch_path_apply<float, float>(contact_, d_wbp_vk.as<double>(), 0, d_y32.as<float>(), d_y32.as<float>(),
-                                        npad_, c, st);
+                                        npad_, c, st, d_wbp_cand.as<int>(), d_wb_count.as<int>());
         launch_st_only<float>(plan32_, d_y32.as<float>(), d_xraw.as<double>(), c, st);
     } else {
         launch_s_only<double>(plan64_, d_vperm64.as<double>(), d_y64.as<double>(), c, st);
@@ -1034,7 +1059,8 @@ void Engine::enqueue_contact_precond(bool f32, bool woodbury, cudaStream_t st) {
                                              d_wbp_u.as<double>(), d_wbp_w.as<double>(), d_wbp_lam.as<double>(),
                                              d_wbp_vk.as<double>(), c, st);
         launch_path_apply<double, double>(contact_, d_wbp_vk.as<double>(), 0, d_y64.as<double>(),
-                                          d_y64.as<double>(), npad_, c, st);
+                                          d_y64.as<double>(), npad_, c, st, d_wbp_cand.as<int>(),
+                                          d_wb_count.as<int>());
         launch_st_only<double>(plan64_, d_y64.as<double>(), d_xraw.as<double>(), c, st);
     }
 }

@@ -271,6 +271,7 @@ private:
     bool build_while_graph(int mode, int cap_iters);
     ContactDev contact_;
     bool has_contact_ = false;
+    bool paths_hold_s_ = false;  // the candidates' column paths hold most of S (mixed-precision contact iteration)
     NodeCsr Acsr_;
     long long launches_ = 0;
     SpmvPlan<double> plan64_;
@@ -308,8 +309,8 @@ private:
     int ws_contact_start_ = 0;
     int* h_ws_err_ = nullptr;    // pinned copy, read after the forward loop's synchronisation
     DeviceBuffer dc_cand, dc_off, dc_prow, dc_pval, dc_G, dc_rprec, dc_lam, dc_lt1, dc_lt2, dc_omega, dc_E, dc_h,
-        dc_act, dc_kact, dc_ainvb, dc_rhs, dc_xsol, dc_bar, dc_M, d_vcon, d_r64, d_q0, dc_Xinv, dc_Xt, dc_pcg,
-        dc_actref, dc_flags, dc_stats, dc_X32, dc_Xt32, dc_refpos, dc_refinv, dc_tprow, dc_tpptr, dc_tpk, dc_tpval,
+        dc_act, dc_kact, dc_ainvb, dc_rhs, dc_xsol, dc_bar, dc_M, d_r64, d_q0, dc_Xinv, dc_Xt, dc_pcg,
+        dc_actref, dc_flags, dc_stats, dc_X32, dc_Xt32, dc_refpos, dc_refinv, dc_tprow, dc_tpdepth, dc_mask, dc_tpptr, dc_tpk, dc_tpval,
         dc_vc;
     Ctrl* h_ctrl_ = nullptr;  // pinned mirror
 };

@@ -6,28 +6,15 @@
 
 #include <algorithm>
 #include <type_traits>
-#include <utility>
 
 #include "kernels.cuh"
+#include "launch.cuh"
 
 namespace dphd {
 
 namespace {
 
 constexpr int kThreads = 256;
-
-// Programmatic dependent launch.  The kernels of an iteration body are launched with programmatic stream
-// serialization (launch_k below), so each grid is launched while its predecessor drains; every such kernel
-// begins with pdl_enter: it lets its own successor launch, then waits (griddepcontrol.wait) until the
-// predecessor grid has completed and its memory is visible, before reading anything.  Launched without the
-// attribute, the wait returns at once.  Every such kernel then reads ctrl->done with an ordinary load (ordered
-// after the wait's memory clobber) and branches on it before it touches data a predecessor wrote: loads through
-// the read-only path (ld.global.nc, which the compiler may treat as invariant and move across the wait) stay
-// behind that branch, so none is issued before the wait.
-__device__ __forceinline__ void pdl_enter() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -512,7 +499,8 @@ __global__ void __launch_bounds__(256) k_spmv_S_units(SpmvPlan<float> p, const f
 
 // y = S v, stage 2: per row, the item partials in item order.
 template <typename T>
-__global__ void __launch_bounds__(kThreads) k_spmv_S_fin(SpmvPlan<T> p, T* __restrict__ y, const Ctrl* ctrl) {
+__global__ void __launch_bounds__(kThreads) k_spmv_S_fin(SpmvPlan<T> p, T* __restrict__ y, float* __restrict__ y32,
+                                                         const Ctrl* ctrl) {
     pdl_enter();
     if (ctrl->done) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -530,6 +518,11 @@ __global__ void __launch_bounds__(kThreads) k_spmv_S_fin(SpmvPlan<T> p, T* __res
         y[i] = s0;
         y[p.npad + i] = s1;
         y[2 * (size_t)p.npad + i] = s2;
+    }
+    if (y32) {
+        y32[i] = (float)s0;
+        y32[p.npad + i] = (float)s1;
+        y32[2 * (size_t)p.npad + i] = (float)s2;
     }
 }
 
@@ -1621,28 +1614,10 @@ __global__ void k_param_reduce(int m, const int* __restrict__ np_k, const int* _
 inline int blocks_for(long long work, int threads) { return (int)((work + threads - 1) / threads); }
 bool g_pdl = true;  // programmatic dependent launch of the iteration-body kernels (process-wide)
 
-// Launches `kern` with programmatic stream serialization when g_pdl is set: the grid may start while its
-// predecessor in the stream drains (the kernel's pdl_enter waits for the predecessor's completion before it
-// reads anything).  Inside stream capture this becomes a programmatic edge of the graph.
-template <typename... KArgs, typename... Args>
-void launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = g_pdl ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
-}
-
-
 }  // namespace
 
 void set_pdl(bool on) { g_pdl = on; }
+bool pdl_enabled() { return g_pdl; }
 
 int device_sms() {
     static int cached[64] = {0};
@@ -1731,7 +1706,7 @@ template <typename T>
 void launch_sts(const SpmvPlan<T>& p, const T* v, T* y, double* x_out, const Ctrl* ctrl, cudaStream_t st) {
     launch_s_items(p, v, ctrl, st);
     if (p.y_accumulate) {
-        launch_k(k_spmv_S_fin<T>, blocks_for(p.n, kThreads), kThreads, 0, st, p, y, ctrl);
+        launch_k(k_spmv_S_fin<T>, blocks_for(p.n, kThreads), kThreads, 0, st, p, y, (float*)nullptr, ctrl);
         launch_st_part<T, false>(p, y, ctrl, st);
     } else {
         launch_st_part<T, true>(p, nullptr, ctrl, st);
@@ -1987,17 +1962,17 @@ void launch_param_reduce(int m, int ne, const int* np_k, const int* type_k, cons
 }
 
 template <typename T>
-void launch_s_only(const SpmvPlan<T>& p, const T* v, T* y, const Ctrl* ctrl, cudaStream_t st) {
+void launch_s_only(const SpmvPlan<T>& p, const T* v, T* y, const Ctrl* ctrl, cudaStream_t st, float* y32) {
     launch_s_items(p, v, ctrl, st);
-    launch_k(k_spmv_S_fin<T>, blocks_for(p.n, kThreads), kThreads, 0, st, p, y, ctrl);
+    launch_k(k_spmv_S_fin<T>, blocks_for(p.n, kThreads), kThreads, 0, st, p, y, y32, ctrl);
 }
 template <typename T>
 void launch_st_only(const SpmvPlan<T>& p, const T* y, double* x_out, const Ctrl* ctrl, cudaStream_t st) {
     launch_st_part<T, false>(p, y, ctrl, st);
     launch_k(k_spmv_ST_fin<T>, blocks_for((long long)p.ntiles * 3 * kTileCols, kThreads), kThreads, 0, st, p, x_out, ctrl);
 }
-template void launch_s_only<double>(const SpmvPlan<double>&, const double*, double*, const Ctrl*, cudaStream_t);
-template void launch_s_only<float>(const SpmvPlan<float>&, const float*, float*, const Ctrl*, cudaStream_t);
+template void launch_s_only<double>(const SpmvPlan<double>&, const double*, double*, const Ctrl*, cudaStream_t, float*);
+template void launch_s_only<float>(const SpmvPlan<float>&, const float*, float*, const Ctrl*, cudaStream_t, float*);
 template void launch_st_only<double>(const SpmvPlan<double>&, const double*, double*, const Ctrl*, cudaStream_t);
 template void launch_st_only<float>(const SpmvPlan<float>&, const float*, double*, const Ctrl*, cudaStream_t);
 

@@ -254,7 +254,7 @@ struct ContactDev {
     int* act_ref = nullptr;
     int* ref_pos = nullptr;
     int* ref_inv = nullptr;
-    int* ncp_flags = nullptr;
+    int* ncp_flags = nullptr;        // 8 words: [0..3] above, [4] k_ncp_prepare's arrival counter
     unsigned long long* ncp_stats = nullptr;
     int cached = 1;                  // 1: the cached-factor solve, 0: a fresh factorisation every PD iteration
     double cg_tol = 1e-13;           // relative residual of the cached-factor CG
@@ -265,11 +265,14 @@ struct ContactDev {
     const int64_t* tp_ptr = nullptr; // nU + 1
     const int* tp_k = nullptr;       // entries: candidate
     const double* tp_val = nullptr;  // entries: S[row, column of the candidate]
+    const int* tp_depth = nullptr;   // nU: position of the row on every path that holds it (its etree depth)
+    long long tp_entries = 0;
+    unsigned int* act_mask = nullptr;  // active flags, one bit per candidate
     double* vc = nullptr;            // 3 K: the S-pass input at the candidates after the NCP step (FP64)
 };
-template <typename T>
-void launch_ncp_cached_solve(const ContactDev& c, const double* q0, const int* iperm, T* vcon, int npad,
-                             const double* r64, Ctrl* ctrl, cudaStream_t st);
+void launch_ncp_cached_solve(const ContactDev& c, const double* q0, const double* r64, Ctrl* ctrl, cudaStream_t st);
+// Active systems of at most this many candidates are solved by one CTA in shared memory (no grid barrier).
+constexpr int kNcpSmall = 64;
 // The preconditioner of the contact-aware adjoint (contact_precond.cu): the three unit directions of the
 // constraint basis, the parts of one application (stage 0: u = J A^-1 r from y = S r, lam = X^T X u per direction
 // block; stage 1: the S-pass input -J^T lam), and the set-up gather of G_b with an identity X_b.
@@ -292,26 +295,25 @@ size_t ncp_matrix_capacity(int K);
 int ncp_grid();
 void launch_delassus(int K, const int64_t* off, const int* prow, const double* pval, double* G, cudaStream_t st);
 // One NCP iteration: y (T) holds S r for the iteration's right-hand side (S b in FP64; S (b - A x) in the
-// FP32 refinement form, where x_base = x adds the current iterate back).  vcon (T) receives J^T f; with r64
-// (FP64 r, refinement form) vcon is the S-pass input and receives r + J^T f at the candidates instead.
-template <typename T>
-void launch_ncp_iteration(const ContactDev& c, const double* x, const T* y, int npad, const double* x_base,
-                          const double* q0, const int* iperm, T* vcon, const double* r64, Ctrl* ctrl,
-                          cudaStream_t st);
+// FP32 refinement form, where x_base = x adds the current iterate back).  c.vc receives J^T f at the candidates;
+// with r64 (FP64 r, refinement form) r + J^T f.
+void launch_ncp_iteration(const ContactDev& c, const double* x, const double* y, int npad, const double* x_base,
+                          const double* q0, const double* r64, Ctrl* ctrl, cudaStream_t st);
 // y_out = y_in + S v at the rows of U, v supported on the candidates (one warp per row, FP64 sums):
-// v_k = v_src[3 cand[k] + d] (node order, from_nodes) or v_src[3 k + d].  y_in may alias y_out.
+// v_k = v_src[3 cand[k] + d] (node order, from_nodes) or v_src[3 k + d].  y_in may alias y_out.  With `list` and
+// `count` (device), v is supported on the `*count` candidates of `list` alone.
 template <typename TI, typename TO>
 void launch_path_apply(const ContactDev& c, const double* v_src, int from_nodes, const TI* y_in, TO* y_out, int npad,
-                       const Ctrl* ctrl, cudaStream_t st);
+                       const Ctrl* ctrl, cudaStream_t st, const int* list = nullptr, const int* count = nullptr);
 // zero the candidates' entries of a permuted S-pass input
 void launch_cand_zero(const ContactDev& c, const int* iperm, float* v, int npad, const Ctrl* ctrl, cudaStream_t st);
 // the values of the row-wise path entries from the column paths (set-up)
 void launch_path_gather_vals(long long E, const int64_t* src_e, const double* pval, double* tp_val, cudaStream_t st);
 void launch_restitution(const ContactDev& c, double* q, const double* q0, const double* v0, double h, double e,
                         double slop, cudaStream_t st);
-// y (+)= S v only (first half of the pair), and x = S^T y only (second half).
+// y (+)= S v only (first half of the pair; with y32 also its FP32 copy), and x = S^T y only (second half).
 template <typename T>
-void launch_s_only(const SpmvPlan<T>& p, const T* v, T* y, const Ctrl* ctrl, cudaStream_t st);
+void launch_s_only(const SpmvPlan<T>& p, const T* v, T* y, const Ctrl* ctrl, cudaStream_t st, float* y32 = nullptr);
 template <typename T>
 void launch_st_only(const SpmvPlan<T>& p, const T* y, double* x_out, const Ctrl* ctrl, cudaStream_t st);
 

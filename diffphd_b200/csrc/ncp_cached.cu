@@ -21,6 +21,7 @@
 #include <cuda_runtime.h>
 
 #include "kernels.cuh"
+#include "ncp_common.cuh"
 
 namespace dphd {
 
@@ -35,11 +36,7 @@ constexpr double kOmegaMin = 1e-6;     // |omega| below this: the candidate's ro
 constexpr double kEDrift = 0.1;        // |E - (omega / omega_ref)^2 E_ref| above this fraction of M_kk: diagonal
 constexpr long long kSpins = 1ll << 24;
 
-__device__ __forceinline__ double wsum(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
+__device__ __forceinline__ double wsum(double v) { return ncp_warp_sum(v); }
 
 __device__ __forceinline__ bool gsync(unsigned int* bar, Ctrl* ctrl) {
     __shared__ int s_ok;
@@ -148,30 +145,68 @@ __device__ __forceinline__ void tile_fma(const double* sA, const double* sB, dou
     }
 }
 
-template <typename T>
+// An active system of at most kNcpSmall candidates, by one CTA: M in shared memory, Cholesky, two triangular solves by
+// one warp, then the multipliers and the cone.  The grid's phases below cost about 5 us per grid barrier (67 us for
+// 3 to 6 active candidates); here a column costs three block barriers.  The cached factor and its list are untouched.
+__device__ void small_solve(const ContactDev& c, int ka, const double* __restrict__ q0, const double* __restrict__ r64,
+                            double* sM) {
+    __shared__ double sx[kNcpSmall];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
+    for (int a = wid; a < ka; a += nw) {
+        const double h = ncp_row(c, a, ka, lane, [&](int b, double m) { sM[a * kLd + b] = m; });
+        if (lane == 0) sx[a] = h;
+    }
+    __syncthreads();
+    for (int j = 0; j < ka; ++j) {
+        const double d = sM[j * kLd + j];
+        const double piv = sqrt(d > 1e-300 ? d : 1e-300), inv = 1.0 / piv;
+        __syncthreads();  // every thread holds the pivot before column j is scaled
+        for (int r = j + tid; r < ka; r += blockDim.x) sM[r * kLd + j] = r == j ? piv : sM[r * kLd + j] * inv;
+        __syncthreads();
+        const int rem = ka - j - 1;
+        for (int t = tid; t < rem * rem; t += blockDim.x) {
+            const int r = j + 1 + t / rem, l = j + 1 + t % rem;
+            if (l <= r) sM[r * kLd + l] -= sM[r * kLd + j] * sM[l * kLd + j];
+        }
+        __syncthreads();
+    }
+    if (wid == 0) {
+        for (int j = 0; j < ka; ++j) {  // L y = rhs
+            if (lane == 0) sx[j] /= sM[j * kLd + j];
+            __syncwarp();
+            const double xj = sx[j];
+            for (int r = j + 1 + lane; r < ka; r += 32) sx[r] -= sM[r * kLd + j] * xj;
+            __syncwarp();
+        }
+        for (int j = ka - 1; j >= 0; --j) {  // L^T x = y
+            if (lane == 0) sx[j] /= sM[j * kLd + j];
+            __syncwarp();
+            const double xj = sx[j];
+            for (int l = lane; l < j; l += 32) sx[l] -= sM[j * kLd + l] * xj;
+            __syncwarp();
+        }
+    }
+    __syncthreads();
+    if (tid < ka) ncp_clamp_row(c, c.act[tid], sx[tid]);
+    __syncthreads();
+    for (int a = wid; a < ka; a += nw) ncp_finish_row(c, a, ka, lane, q0, r64);
+}
+
 __global__ void __launch_bounds__(kThr, 1)
-k_ncp_cached_solve(ContactDev c, const double* __restrict__ q0, const int* __restrict__ iperm, T* __restrict__ vcon,
-                   int npad, const double* __restrict__ r64, Ctrl* ctrl) {
+k_ncp_cached_solve(ContactDev c, const double* __restrict__ q0, const double* __restrict__ r64, Ctrl* ctrl) {
     extern __shared__ double smem[];
     double* sD = smem;
     double* sA = smem + kT * kLd;
     double* sB = smem + 2 * kT * kLd;
     if (ctrl->done) return;
-    const int K = c.K, ka = c.kact[0];
+    const int ka = c.kact[0];
     const int tid = threadIdx.x, nt = blockDim.x, G = gridDim.x, bid = blockIdx.x;
     const int gt = bid * nt + tid, nthr = G * nt;
     const int lane = tid & 31, gw = gt >> 5, nwarps = nthr >> 5;
-    const double n0 = c.n[0], n1 = c.n[1], n2 = c.n[2];
     const int ldx = (int)c.kcap;
-    for (int k = gt; k < K; k += nthr) {
-        const int node = c.cand[k], j = iperm[node];
-        vcon[j] = r64 ? (T)r64[3 * node] : T(0);
-        vcon[npad + j] = r64 ? (T)r64[3 * node + 1] : T(0);
-        vcon[2 * (size_t)npad + j] = r64 ? (T)r64[3 * node + 2] : T(0);
-        for (int d = 0; d < 3; ++d) c.vc[3 * (size_t)k + d] = r64 ? r64[3 * node + d] : 0.0;
-    }
-    if (ka == 0) {
-        for (int k = gt; k < K; k += nthr) c.lt1[k] = c.lt2[k] = 0.0;
+    if (ka == 0) return;
+    if (ka <= kNcpSmall) {  // the same in every CTA: no grid barrier is reached
+        if (bid == 0) small_solve(c, ka, q0, r64, smem);
         return;
     }
     const int nb = (ka + kT - 1) / kT, ld = nb * kT;
@@ -201,34 +236,12 @@ k_ncp_cached_solve(ContactDev c, const double* __restrict__ q0, const int* __res
         }
         const int k = c.act[a];
         if (have && lane == 0 && c.ref_pos[k] < 0) ++n_new_w;
-        const double om = c.omega[k];
-        const double* Gk = c.G + (size_t)k * K;
-        double g0 = 0.0, g1 = 0.0, g2 = 0.0;
-        for (int b = lane; b < ld; b += 32) {
-            if (b >= ka) {
-                Ma[b] = 0.0;
-                continue;
-            }
-            const int kb = c.act[b];
-            const double Gab = Gk[kb];
-            const double fn = c.omega[kb] * c.lam[kb];
-            const double f1 = c.lt1[kb], f2 = c.lt2[kb];
-            g0 += Gab * (fn * n0 + f1 * c.t1[0] + f2 * c.t2[0]);
-            g1 += Gab * (fn * n1 + f1 * c.t1[1] + f2 * c.t2[1]);
-            g2 += Gab * (fn * n2 + f1 * c.t1[2] + f2 * c.t2[2]);
-            const double m = om * Gab * c.omega[kb] + (a == b ? c.Ediag[k] : 0.0);
+        const double h = ncp_row(c, a, ka, lane, [&](int b, double m) {
             Ma[b] = m;
             if (a == b) dg[a] = m;
-        }
-        g0 = wsum(g0);
-        g1 = wsum(g1);
-        g2 = wsum(g2);
-        if (lane == 0) {
-            g0 += c.ainvb[3 * a];
-            g1 += c.ainvb[3 * a + 1];
-            g2 += c.ainvb[3 * a + 2];
-            rhs[a] = c.hvec[k] - om * (n0 * g0 + n1 * g1 + n2 * g2);
-        }
+        });
+        for (int b = ka + lane; b < ld; b += 32) Ma[b] = 0.0;
+        if (lane == 0) rhs[a] = h;
     }
     if (n_new_w) atomicAdd(flags + 2, n_new_w);
     if (!gsync(c.bar, ctrl)) return;
@@ -366,7 +379,7 @@ k_ncp_cached_solve(ContactDev c, const double* __restrict__ q0, const int* __res
     if (!solved) {
         // ---- C: blocked Cholesky of M with X = L^-1 (identity solved in place), then x = X^T X rhs ----
         double* X = c.Xinv;
-        for (int k = gt; k < K; k += nthr) c.ref_pos[k] = -1;  // read no more in this launch (after its CG)
+        for (int k = gt; k < c.K; k += nthr) c.ref_pos[k] = -1;  // read no more in this launch (after its CG)
         for (size_t e = (size_t)gt; e < (size_t)ld * ld; e += (size_t)nthr) {
             const int a = (int)(e / ld), b = (int)(e % ld);
             X[(size_t)a * ldx + b] = a == b ? 1.0 : 0.0;
@@ -539,83 +552,16 @@ k_ncp_cached_solve(ContactDev c, const double* __restrict__ q0, const int* __res
     if (!gsync(c.bar, ctrl)) return;
     if (gt == 0) flags[2] = 0;  // re-armed for the next launch
     // ---- D: multipliers, Coulomb cone, contact right-hand side ----
-    for (int a = gt; a < ka; a += nthr) {
-        const int k = c.act[a];
-        double l = c.lam[k] + x[a];
-        l = l < 0.0 ? 0.0 : (l > 1e8 ? 1e8 : l);
-        c.lam[k] = l;
-    }
-    for (int k = gt; k < K; k += nthr) c.lt1[k] = c.lt2[k] = 0.0;
+    for (int a = gt; a < ka; a += nthr) ncp_clamp_row(c, c.act[a], x[a]);
     if (!gsync(c.bar, ctrl)) return;
-    for (int a = gw; a < ka; a += nwarps) {
-        const int k = c.act[a];
-        double t1v = 0.0, t2v = 0.0;
-        if (c.mu > 0.0 && c.lam[k] > 0.0) {
-            const double* Gk = c.G + (size_t)k * K;
-            double f = 0.0;
-            for (int b = lane; b < ka; b += 32) {
-                const int kb = c.act[b];
-                f += c.omega[kb] * c.lam[kb] * Gk[kb];
-            }
-            f = wsum(f);
-            const int node = c.cand[k];
-            const double qn0 = c.ainvb[3 * a] + f * n0, qn1 = c.ainvb[3 * a + 1] + f * n1,
-                         qn2 = c.ainvb[3 * a + 2] + f * n2;
-            const double s0 = qn0 - q0[3 * node], s1 = qn1 - q0[3 * node + 1], s2 = qn2 - q0[3 * node + 2];
-            const double sn = s0 * n0 + s1 * n1 + s2 * n2;
-            const double u0 = s0 - sn * n0, u1 = s1 - sn * n1, u2 = s2 - sn * n2;
-            const double ut1 = u0 * c.t1[0] + u1 * c.t1[1] + u2 * c.t1[2];
-            const double ut2 = u0 * c.t2[0] + u1 * c.t2[1] + u2 * c.t2[2];
-            const double Gkk = Gk[k];
-            double st1 = 0.0, st2 = 0.0;
-            if (fabs(Gkk * Gkk) > 1e-20) {
-                st1 = -ut1 / Gkk;
-                st2 = -ut2 / Gkk;
-            }
-            const double cone = c.mu * c.lam[k];
-            if (sqrt(st1 * st1 + st2 * st2) <= cone + 1e-14) {
-                t1v = st1;
-                t2v = st2;
-            } else {
-                const double um = sqrt(ut1 * ut1 + ut2 * ut2);
-                if (um > 1e-14) {
-                    t1v = -cone * ut1 / um;
-                    t2v = -cone * ut2 / um;
-                }
-            }
-        }
-        if (lane == 0) {
-            c.lt1[k] = t1v;
-            c.lt2[k] = t2v;
-            const double fn = c.omega[k] * c.lam[k];
-            const int node = c.cand[k], j = iperm[node];
-            const double r0 = r64 ? r64[3 * node] : 0.0, r1 = r64 ? r64[3 * node + 1] : 0.0,
-                         r2 = r64 ? r64[3 * node + 2] : 0.0;
-            const double w0 = r0 + fn * n0 + t1v * c.t1[0] + t2v * c.t2[0];
-            const double w1 = r1 + fn * n1 + t1v * c.t1[1] + t2v * c.t2[1];
-            const double w2 = r2 + fn * n2 + t1v * c.t1[2] + t2v * c.t2[2];
-            vcon[j] = (T)w0;
-            vcon[npad + j] = (T)w1;
-            vcon[2 * (size_t)npad + j] = (T)w2;
-            c.vc[3 * (size_t)k] = w0;
-            c.vc[3 * (size_t)k + 1] = w1;
-            c.vc[3 * (size_t)k + 2] = w2;
-        }
-    }
+    for (int a = gw; a < ka; a += nwarps) ncp_finish_row(c, a, ka, lane, q0, r64);
 }
 
 }  // namespace
 
-template <typename T>
-void launch_ncp_cached_solve(const ContactDev& c, const double* q0, const int* iperm, T* vcon, int npad,
-                             const double* r64, Ctrl* ctrl, cudaStream_t st) {
+void launch_ncp_cached_solve(const ContactDev& c, const double* q0, const double* r64, Ctrl* ctrl, cudaStream_t st) {
     const size_t smem = (size_t)(3 * kT * kLd) * sizeof(double);
-    static bool attr_set[2] = {false, false};
-    void (*kern)(ContactDev, const double*, const int*, T*, int, const double*, Ctrl*) = k_ncp_cached_solve<T>;
-    if (!attr_set[sizeof(T) == 8]) {
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        attr_set[sizeof(T) == 8] = true;
-    }
+    cudaFuncSetAttribute(k_ncp_cached_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ncp_grid());
     cfg.blockDim = dim3(kThr);
@@ -626,11 +572,7 @@ void launch_ncp_cached_solve(const ContactDev& c, const double* q0, const int* i
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kern, c, q0, iperm, vcon, npad, r64, ctrl);
+    cudaLaunchKernelEx(&cfg, k_ncp_cached_solve, c, q0, r64, ctrl);
 }
-template void launch_ncp_cached_solve<double>(const ContactDev&, const double*, const int*, double*, int,
-                                              const double*, Ctrl*, cudaStream_t);
-template void launch_ncp_cached_solve<float>(const ContactDev&, const double*, const int*, float*, int,
-                                             const double*, Ctrl*, cudaStream_t);
 
 }  // namespace dphd
