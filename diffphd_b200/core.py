@@ -471,7 +471,7 @@ class Deformable:
         self._check(self._L.dphd_debug_set_pdl(self._h, int(bool(on))))
 
     def set_s_kernel(self, row_groups=True):
-        """FP32 y = S v pass: one warp per row group or one warp per row segment (bit-identical sums; by default
+        """y = S v pass: one warp per row group or one warp per row segment (bit-identical sums; by default
         the faster one is picked by timing both when the factor is built)."""
         self._check(self._L.dphd_debug_set_s_kernel(self._h, int(bool(row_groups))))
 

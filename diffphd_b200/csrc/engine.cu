@@ -344,6 +344,8 @@ void Engine::build_device(int threads) {
     // share their first column (one separator) are emitted row-fastest so one CTA reads one slice of v.
     // The items of one group and segment form one unit of the row-group kernel (first item, rows, first column,
     // widest row's columns).
+    const StsSizes sizes = sts_sizes((long long)ro[n]);
+    const int seg_cols = sizes.seg_cols;
     std::vector<int> it_row, it_c0, it_nc;
     std::vector<int4> units;
     for (int i = 0; i < n;) {
@@ -351,14 +353,14 @@ void Engine::build_device(int threads) {
         while (j < n && ra[j] == ra[i] && j - i < kUnitRows) ++j;
         int glen = 0;
         for (int r = i; r < j; ++r) glen = std::max(glen, rl[r]);
-        for (int c0 = 0; c0 < glen; c0 += kSegCols) {
+        for (int c0 = 0; c0 < glen; c0 += seg_cols) {
             const int first = (int)it_row.size();
             int ncmax = 0;
             for (int r = i; r < j; ++r)
                 if (c0 < rl[r]) {
                     it_row.push_back(r);
                     it_c0.push_back(c0);
-                    it_nc.push_back(std::min(kSegCols, rl[r] - c0));
+                    it_nc.push_back(std::min(seg_cols, rl[r] - c0));
                     ncmax = std::max(ncmax, it_nc.back());
                 }
             units.push_back(make_int4(first, (int)it_row.size() - first, ra[i] + c0, ncmax));
@@ -372,10 +374,17 @@ void Engine::build_device(int threads) {
         std::vector<int> pos(r_ptr.begin(), r_ptr.end() - 1);
         for (size_t t = 0; t < it_row.size(); ++t) r_items[pos[it_row[t]]++] = (int)t;
     }
-    // x = S^T y schedule: each tile's row list in chunks of `chunk` rows (long chunks for large factors, where
-    // they keep more bytes in flight per CTA; short ones for small factors, where they make enough CTAs)
-    const int chunk = st_chunk_rows_ > 0 ? st_chunk_rows_ : ((long long)ro[n] > kChunkLargeValues ? kChunkRows
-                                                                                                  : kChunkRowsSmall);
+    // x = S^T y schedule: each tile's row list in chunks of `chunk` rows
+    const int chunk = st_chunk_rows_ > 0 ? st_chunk_rows_ : sizes.chunk_rows;
+    // The allocation-free entry point accepts the meshes whose partial sums fit its scratch with 2,048-column items and
+    // 64-row chunks (512 above 2^28 values), whatever schedule this factor gets.
+    size_t scratch_items = 0, scratch_chunks = 0;
+    {
+        const int cap_rows = (long long)ro[n] > (1ll << 28) ? 512 : 64;
+        for (int i = 0; i < n; ++i) scratch_items += (size_t)(rl[i] + 2047) / 2048;
+        for (int t = 0; t < ntiles_; ++t)
+            scratch_chunks += (size_t)std::max(1, (tcnt[t + 1] - tcnt[t] + cap_rows - 1) / cap_rows);
+    }
     std::vector<int> c_tile, c_p0, c_p1, t_cptr(ntiles_ + 1, 0);
     for (int t = 0; t < ntiles_; ++t) {
         for (int p0 = tcnt[t]; p0 < tcnt[t + 1]; p0 += chunk) {
@@ -485,7 +494,9 @@ void Engine::build_device(int threads) {
         P.row_item_ptr = d_row_item_ptr.as<int>();
         P.row_items = d_row_items.as<int>();
         P.n_chunks = (int)c_tile.size();
-        P.st_rows = st_rows_;
+        P.st_rows = st_chunk_rows_ > 0 ? st_rows_ : sizes.st_rows;
+        P.scratch_items = scratch_items;
+        P.scratch_chunks = scratch_chunks;
         P.ntiles = ntiles_;
         P.chunk_tile = d_chunk_tile.as<int>();
         P.chunk_p0 = d_chunk_p0.as<int>();
@@ -506,20 +517,20 @@ void Engine::build_device(int threads) {
     // the factor stays in L2 across PD iterations when it takes at most about half of it (126 MB on B200)
     plan64_.keep_in_l2 = d_vals64.bytes <= (64ull << 20) ? 1 : 0;
     plan32_.keep_in_l2 = d_vals32.bytes <= (64ull << 20) ? 1 : 0;
-    plan32_.n_units = (int)units.size();
-    plan32_.unit_desc = d_unit_desc.as<int4>();
-    plan32_.unit_item_desc = d_unit_item_desc.as<int4>();
-    plan32_.unit_item_rslots = d_unit_item_rslots.as<int2>();
-    for (auto* P : {&plan32_}) {
-        P->yrow = d_yrow32.as<float>();
-        P->row_cnt = d_row_cnt.as<unsigned int>();
-        P->item_rslots = d_item_rslots.as<int2>();
-    }
-    plan64_.yrow = d_yrow64.as<double>();
-    plan64_.row_cnt = d_row_cnt.as<unsigned int>();
-    plan64_.item_rslots = d_item_rslots.as<int2>();
-    plan32_.unit_item_slot = d_unit_item_slot.as<int>();
-    plan32_.use_units = s_units_ ? 1 : 0;
+    auto fill_units = [&](auto& P, DeviceBuffer& yrow, bool use) {
+        using T = std::remove_const_t<std::remove_pointer_t<decltype(P.vals)>>;
+        P.n_units = (int)units.size();
+        P.unit_desc = d_unit_desc.as<int4>();
+        P.unit_item_desc = d_unit_item_desc.as<int4>();
+        P.unit_item_rslots = d_unit_item_rslots.as<int2>();
+        P.unit_item_slot = d_unit_item_slot.as<int>();
+        P.yrow = yrow.template as<T>();
+        P.row_cnt = d_row_cnt.as<unsigned int>();
+        P.item_rslots = d_item_rslots.as<int2>();
+        P.use_units = use ? 1 : 0;
+    };
+    fill_units(plan64_, d_yrow64, false);
+    fill_units(plan32_, d_yrow32, false);
     // mesh, samples, constraints
     dE.upload(M.E);
     dX.upload(M.X);
@@ -588,30 +599,34 @@ void Engine::build_device(int threads) {
     CUDA_OK(cudaMemset(d_y32.p, 0, d_y32.bytes));
     d_ctrl.alloc(sizeof(Ctrl));
     CUDA_OK(cudaMemset(d_ctrl.p, 0, sizeof(Ctrl)));
-    // The two FP32 y = S v kernels (one warp per row segment, one warp per row group) give bit-identical sums
-    // (the same per-lane order); which is faster depends on the factor's shape, so both are timed once here on
-    // this factor (a warm-up and 5 launches each) and the faster one is kept.
+    // The two y = S v kernels (one warp per row segment, one warp per row group) give bit-identical sums (the same
+    // per-lane order); which is faster depends on the factor's shape, so both are timed once here on this factor in
+    // each precision (a warm-up and 5 launches each) and the faster one is kept.
     {
         cudaEvent_t e0, e1;
         CUDA_OK(cudaEventCreate(&e0));
         CUDA_OK(cudaEventCreate(&e1));
-        float ms[2] = {0.f, 0.f};
         const Ctrl* c = d_ctrl.as<Ctrl>();
-        for (int which = 0; which < 2; ++which) {
-            SpmvPlan<float> p = plan32_;
-            p.use_units = which;
-            launch_s_only<float>(p, d_vperm32.as<float>(), d_y32.as<float>(), c, stream_);
-            CUDA_OK(cudaEventRecord(e0, stream_));
-            for (int r = 0; r < 5; ++r) launch_s_only<float>(p, d_vperm32.as<float>(), d_y32.as<float>(), c, stream_);
-            CUDA_OK(cudaEventRecord(e1, stream_));
-            CUDA_OK(cudaEventSynchronize(e1));
-            CUDA_OK(cudaEventElapsedTime(&ms[which], e0, e1));
-        }
+        auto pick = [&](auto& plan, const auto* v, auto* y) {
+            using T = std::remove_pointer_t<decltype(y)>;
+            float ms[2] = {0.f, 0.f};
+            for (int which = 0; which < 2; ++which) {
+                auto p = plan;
+                p.use_units = which;
+                launch_s_only<T>(p, v, y, c, stream_);
+                CUDA_OK(cudaEventRecord(e0, stream_));
+                for (int r = 0; r < 5; ++r) launch_s_only<T>(p, v, y, c, stream_);
+                CUDA_OK(cudaEventRecord(e1, stream_));
+                CUDA_OK(cudaEventSynchronize(e1));
+                CUDA_OK(cudaEventElapsedTime(&ms[which], e0, e1));
+            }
+            plan.use_units = ms[1] < ms[0] ? 1 : 0;
+            launches_ += 24;
+        };
+        pick(plan32_, d_vperm32.as<float>(), d_y32.as<float>());
+        pick(plan64_, d_vperm64.as<double>(), d_y64.as<double>());
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
-        s_units_ = ms[1] < ms[0];
-        plan32_.use_units = s_units_ ? 1 : 0;
-        launches_ += 24;
     }
     double gf[3] = {0, 0, 0};
     if (M.has_gravity)
@@ -1367,8 +1382,7 @@ void Engine::forward_device_init(const double* dq, const double* dv, const doubl
 
 void Engine::set_s_units(bool on) {
     drop_graphs();
-    s_units_ = on;
-    plan32_.use_units = on ? 1 : 0;
+    plan32_.use_units = plan64_.use_units = on ? 1 : 0;
 }
 
 double Engine::ws_dx() const { return std::pow(M.vol, 1.0 / 3.0); }

@@ -152,8 +152,8 @@ public:
     // (set = false) or from (set = true) a device array of 2 * 3n doubles, so that a checkpointed rollout can
     // recompute a segment exactly as the forward pass ran it
     void ws_state(double* d_buf, int* valid, bool set, cudaStream_t st);
-    // selects the row-group or the one-warp-per-item kernel of the FP32 y = S v pass (overriding the choice
-    // timed at factor build); drops the captured iteration graphs
+    // selects the row-group or the one-warp-per-item kernel of the y = S v pass (overriding the choice timed at
+    // factor build); drops the captured iteration graphs
     void set_s_units(bool on);
     void drop_captured_graphs() { drop_graphs(); }
 
@@ -293,7 +293,6 @@ private:
     DeviceBuffer d_item_desc, d_item_slot, d_trow_desc, d_trow_off, d_J32;
     DeviceBuffer d_unit_desc, d_unit_item_desc, d_unit_item_slot;  // row-group units of the FP32 y = S v pass
     DeviceBuffer d_item_rslots, d_unit_item_rslots, d_row_cnt, d_yrow32, d_yrow64;  // multi-item row totals
-    bool s_units_ = false;       // chosen by timing both kernels when the factor is built
     DeviceBuffer d_gq, d_gv, d_dq, d_dv, d_df, d_A_rp, d_A_ci, d_A_v, d_r, d_pp, d_wv, d_wlog, d_mu_prev;
     bool mu_prev_valid_ = false, mu_prev2_valid_ = false, mu_prev3_valid_ = false, mu_prev4_valid_ = false;
     DeviceBuffer d_mu_prev2, d_mu_prev3, d_mu_prev4;  // the adjoints before d_mu_prev (bwd_warm_start 2-4)

@@ -341,10 +341,19 @@ __device__ __forceinline__ void row_arrive(const SpmvPlan<T>& p, int z, int w) {
     p.row_cnt[z] = 0u;  // ready for the next apply
     __threadfence();
     T s0 = T(0), s1 = T(0), s2 = T(0);
-    for (int k = z; k < w; ++k) {
-        s0 += __ldcg(p.ypart + 3 * (size_t)k);
-        s1 += __ldcg(p.ypart + 3 * (size_t)k + 1);
-        s2 += __ldcg(p.ypart + 3 * (size_t)k + 2);
+    for (int k = z; k < w; k += 8) {  // eight slots' loads in flight, added in slot order
+        T t[8][3];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) t[u][d] = k + u < w ? __ldcg(p.ypart + 3 * (size_t)(k + u) + d) : T(0);
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (k + u < w) {
+                s0 += t[u][0];
+                s1 += t[u][1];
+                s2 += t[u][2];
+            }
     }
     T* o = p.yrow + 3 * (size_t)z;
     o[0] = s0;
@@ -352,7 +361,7 @@ __device__ __forceinline__ void row_arrive(const SpmvPlan<T>& p, int z, int w) {
     o[2] = s2;
 }
 
-// y = S v, stage 1: one warp per work item (a row segment of <= kSegCols columns), four 16-byte loads of S
+// y = S v, stage 1: one warp per work item (a row segment of one schedule segment's columns), four 16-byte loads of S
 // in flight per lane, v through L1 (the CTA's warps share the segment's columns).
 template <typename T>
 __device__ __forceinline__ void s_items_body(const SpmvPlan<T>& p, const T* __restrict__ v, int vb, const Ctrl* ctrl) {
@@ -418,24 +427,30 @@ __global__ void __launch_bounds__(256) k_spmv_S_items(SpmvPlan<T> p, const T* __
     s_items_body(p, v, blockIdx.x, ctrl);
 }
 
-// y = S v, stage 1 by row groups (FP32): one warp per unit (up to kUnitRows rows of one nested-dissection
-// group over one column segment).  Each lane loads the three float4 of v at its columns once and the float4
-// of S of every row of the unit, so v is read once per unit instead of once per row, and every lane keeps up to
-// kUnitRows + 3 independent 16-byte loads in flight.  Rows shorter than the unit's widest row are masked per
-// float4 (row lengths and segment starts are multiples of 4).  Partial sums go to the rows' item slots.
-__global__ void __launch_bounds__(256) k_spmv_S_units(SpmvPlan<float> p, const float* __restrict__ v,
-                                                      const Ctrl* ctrl) {
+// y = S v, stage 1 by row groups: one warp per kWarpRows rows of a unit (up to kUnitRows rows of one
+// nested-dissection group over one column segment).  Each lane loads the vectors of v at its columns once and the
+// vector of S of every row, so v is read once per kWarpRows rows instead of once per row.  What bounds it is the loads
+// in flight: 4 rows a warp keep 114 registers in FP64 (four 128-thread CTAs an SM); 8 rows take 186 and 2 rows read v
+// too often.  The pair on 224 M FP64 values (64x32x32 cantilever): one warp per item 808 us, 8 rows 663, 4 rows 602
+// (5.96 TB/s, 0.91 of the measured copy), 2 rows 703.  Rows shorter than the unit's widest row are masked per vector
+// (row lengths and segment starts are multiples of 4).  Partial sums go to the rows' item slots.
+template <typename T>
+__global__ void __launch_bounds__(128) k_spmv_S_units(SpmvPlan<T> p, const T* __restrict__ v, const Ctrl* ctrl) {
+    constexpr int R = kWarpRows;
     pdl_enter();
     const int done = ctrl->done;  // in flight together with the unit descriptor, tested after it
-    const int u = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    constexpr int kParts = kUnitRows / R;
+    const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    const int u = w / kParts, r0 = (w % kParts) * R;
     if (u >= p.n_units) return;
     const int4 ud = __ldg(p.unit_desc + u);
     if (done) return;
-    const int first = ud.x, nr = ud.y, a = ud.z, ncmax = ud.w;
-    const float* sp[kUnitRows];
-    int nc[kUnitRows];
+    const int nr = min(R, ud.y - r0), first = ud.x + r0, a = ud.z, ncmax = ud.w;
+    if (nr <= 0) return;
+    const T* sp[R];
+    int nc[R];
 #pragma unroll
-    for (int r = 0; r < kUnitRows; ++r) {
+    for (int r = 0; r < R; ++r) {
         sp[r] = p.vals;
         nc[r] = 0;
         if (r < nr) {
@@ -445,48 +460,47 @@ __global__ void __launch_bounds__(256) k_spmv_S_units(SpmvPlan<float> p, const f
         }
     }
     const size_t npad = (size_t)p.npad;
-    const float* v0 = v + a;
-    const float* v1 = v + npad + a;
-    const float* v2 = v + 2 * npad + a;
-    float acc[kUnitRows][3];
+    const T* v0 = v + a;
+    const T* v1 = v + npad + a;
+    const T* v2 = v + 2 * npad + a;
+    T acc[R][3];
 #pragma unroll
-    for (int r = 0; r < kUnitRows; ++r) acc[r][0] = acc[r][1] = acc[r][2] = 0.f;
+    for (int r = 0; r < R; ++r) acc[r][0] = acc[r][1] = acc[r][2] = T(0);
     for (int c = lane * 4; c < ncmax; c += 128) {
-        Vec4<float> x0, x1, x2, sv[kUnitRows];
+        Vec4<T> x0, x1, x2, sv[R];
         x0.load(v0 + c);
         x1.load(v1 + c);
         x2.load(v2 + c);
 #pragma unroll
-        for (int r = 0; r < kUnitRows; ++r) {
+        for (int r = 0; r < R; ++r)
             if (c < nc[r]) sv[r].load_s(sp[r] + c, p.keep_in_l2);
-            else sv[r].v[0] = sv[r].v[1] = sv[r].v[2] = sv[r].v[3] = 0.f;
-        }
 #pragma unroll
-        for (int r = 0; r < kUnitRows; ++r)
+        for (int r = 0; r < R; ++r)
+            if (c < nc[r])
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                acc[r][0] += sv[r].v[q] * x0.v[q];
-                acc[r][1] += sv[r].v[q] * x1.v[q];
-                acc[r][2] += sv[r].v[q] * x2.v[q];
-            }
+                for (int q = 0; q < 4; ++q) {
+                    acc[r][0] += sv[r].v[q] * x0.v[q];
+                    acc[r][1] += sv[r].v[q] * x1.v[q];
+                    acc[r][2] += sv[r].v[q] * x2.v[q];
+                }
     }
 #pragma unroll
-    for (int r = 0; r < kUnitRows; ++r)
+    for (int r = 0; r < R; ++r)
         if (r < nr) {
             acc[r][0] = warp_sum(acc[r][0]);
             acc[r][1] = warp_sum(acc[r][1]);
             acc[r][2] = warp_sum(acc[r][2]);
         }
     if (lane < nr) {  // lane r stores row r's partial (the values are warp-uniform after the sums)
-        float o0 = 0.f, o1 = 0.f, o2 = 0.f;
+        T o0 = T(0), o1 = T(0), o2 = T(0);
 #pragma unroll
-        for (int r = 0; r < kUnitRows; ++r)
+        for (int r = 0; r < R; ++r)
             if (r == lane) {
                 o0 = acc[r][0];
                 o1 = acc[r][1];
                 o2 = acc[r][2];
             }
-        float* o = p.ypart + (size_t)__ldg(p.unit_item_slot + first + lane) * 3;
+        T* o = p.ypart + (size_t)__ldg(p.unit_item_slot + first + lane) * 3;
         o[0] = o0;
         o[1] = o1;
         o[2] = o2;
@@ -1690,14 +1704,13 @@ static void launch_st_part(const SpmvPlan<T>& p, const T* y, const Ctrl* ctrl, c
     else launch_k(k_spmv_ST_part<T, FROM_ITEMS, 4>, p.n_chunks, 256, 0, st, p, y, ctrl);
 }
 
-// stage 1 of y = S v: the row-group kernel for FP32 factors with a unit schedule, else one warp per item
+// stage 1 of y = S v: row groups, or one warp per item
 template <typename T>
 static void launch_s_items(const SpmvPlan<T>& p, const T* v, const Ctrl* ctrl, cudaStream_t st) {
-    if constexpr (std::is_same<T, float>::value) {
-        if (p.use_units && p.n_units > 0) {
-            launch_k(k_spmv_S_units, blocks_for((long long)p.n_units * 32, 256), 256, 0, st, p, v, ctrl);
-            return;
-        }
+    if (p.use_units && p.n_units > 0) {
+        const long long warps = (long long)p.n_units * (kUnitRows / kWarpRows);
+        launch_k(k_spmv_S_units<T>, blocks_for(warps * 32, 128), 128, 0, st, p, v, ctrl);
+        return;
     }
     launch_k(k_spmv_S_items<T>, blocks_for((long long)p.n_items * 32, 256), 256, 0, st, p, v, ctrl);
 }

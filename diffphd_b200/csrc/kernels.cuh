@@ -77,7 +77,7 @@ struct SpmvPlan {
     const int* row_len = nullptr;
     const T* vals = nullptr;
     int keep_in_l2 = 0;  // S fits comfortably in L2: ordinary cached loads instead of evict-first streaming
-    // y = S v: work items (row, first column, column count) of at most kSegCols columns, one warp each;
+    // y = S v: work items (row, first column, column count) of at most one segment's columns, one warp each;
     // items of the same nested-dissection separator and column segment are adjacent so that the warps of
     // one CTA read the same slice of v (L1 reuse).  Partial sums ypart[item][3] are summed per row in item
     // order by the fix-up kernel (rows own items [row_item_ptr[r], row_item_ptr[r+1]) via row_items).
@@ -105,9 +105,9 @@ struct SpmvPlan {
     const int* perm = nullptr;
     const double* x_base = nullptr;  // when set, x_out = x_base + S^T S v (refinement form)
     int y_accumulate = 0;            // when set, y += S v instead of y = S v
-    // y = S v by row groups (FP32 factors): unit u = the items of one group of at most kUnitRows rows that
-    // share a column segment (unit_desc: first item, rows, first column, widest row's columns); one warp
-    // reads the segment of v once for all rows.  use_units = 0 selects the one-warp-per-item kernel.
+    // y = S v by row groups: unit u = the items of one group of at most kUnitRows rows that share a column segment
+    // (unit_desc: first item, rows, first column, widest row's columns); one warp reads the segment of v once for
+    // kWarpRows of them.  use_units = 0 selects the one-warp-per-item kernel.
     // Rows cut into several items: the warp whose item of such a row finishes last sums the row's slot
     // partials in slot order into yrow[3 z] (z = the row's first slot), so that the S^T pass reads one value
     // per row.  item_rslots / unit_item_rslots: (first slot, end slot) of each item's row, in the launch order
@@ -121,13 +121,28 @@ struct SpmvPlan {
     const int4* unit_desc = nullptr;
     const int4* unit_item_desc = nullptr;  // the items in emission order (a unit's rows are consecutive here)
     const int* unit_item_slot = nullptr;
+    size_t scratch_items = 0, scratch_chunks = 0;  // items and chunks the fixed-scratch entry's capacity is stated in
 };
-constexpr int kSegCols = 2048;       // columns per S v work item
-constexpr int kUnitRows = 8;         // rows per S v unit (the row-group cap of the item schedule)
-constexpr int kChunkRows = 512;      // rows per S^T chunk CTA for large factors (64^3 contact block: 64 -> 512
-                                     // rows took the FP32 pair from 4.05 to 3.60 ms)
-constexpr int kChunkRowsSmall = 64;  // for factors of at most kChunkLargeValues values (more CTAs to fill the GPU)
-constexpr long long kChunkLargeValues = 1ll << 28;
+// Schedule by the factor's size (padded values).  Long segments and chunks keep more bytes in flight per warp and CTA
+// and leave fewer partial sums; short ones make enough of them to fill the GPU.  Pair times in us, FP64 / FP32:
+//   54 M (48x24x24 hexes)           segment 1,024: 177 / 100   2,048: 167 / 95      4,096: 169 / 98
+//                                   chunk 64: 223 / 107        192: 210 / 99        512: 213 / 105
+//   224 M (64x32x32 hexes)          segment 2,048: 624 / 338   4,096: 602 / 324     8,192: 601 / 336
+//                                   chunk 64: 903 / 396        192: 827 / 353       512: 812 / 345
+// At 7.3 M (32x16x16 tets) 1,024-column segments would save 5% of the pair, but the sums' order is part of what a
+// contact-free FP64 rollout that stops at a loose gate returns, and there it stays as it is.
+struct StsSizes {
+    int seg_cols;    // columns per S v work item
+    int chunk_rows;  // rows per S^T chunk CTA
+    int st_rows;     // rows in flight per warp of the S^T pass
+};
+constexpr StsSizes sts_sizes(long long values) {
+    return values <= (16ll << 20)    ? StsSizes{2048, 64, 4}
+           : values <= (128ll << 20) ? StsSizes{2048, 192, 4}
+                                     : StsSizes{4096, 512, 8};
+}
+constexpr int kUnitRows = 8;  // rows per S v unit (the row-group cap of the item schedule)
+constexpr int kWarpRows = 4;  // rows of a unit per warp
 constexpr int kStChunkMax = 512;     // largest S^T chunk (its row descriptors are staged in shared memory)
 constexpr int kGatherLanes = 8;      // lanes per node in the node gathers
 constexpr int kGatherMaxThreads = 512;  // block-size bound of the node gathers
