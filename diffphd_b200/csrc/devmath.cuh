@@ -322,11 +322,20 @@ __device__ __forceinline__ bool project_delta(int type, T mu, T la, T k, const T
     return ok;
 }
 
-// Directional derivative of Bp along dF (corotated: dR from the 3x3 system of geometry.cpp:60-80;
-// volume: KKT system of volume_pd_element_energy.cpp:61-155; Neo-Hookean: implicit function theorem on the
-// proximal optimality, neohookean_pd_element_energy.cpp:133-165).
+// What the directional derivatives of one energy share at a sample: the volume projection's D = sig* - sig (type 1) or
+// the Neo-Hookean proximal point (type 2), both iterative.
 template <typename T>
-__device__ void project_diff(int type, T mu, T la, T k, const T* U, const T* sig, const T* V, const T* dF, T* out) {
+__device__ __forceinline__ void project_point(int type, T mu, T la, T k, const T* sig, T* s) {
+    if (type == 1) volume_D(sig, s);
+    else if (type == 2) nh_prox(mu, la, k, sig, s);
+}
+
+// Directional derivative of Bp along dF at the sample's project_point `sp` (corotated: dR from the 3x3 system of
+// geometry.cpp:60-80; volume: KKT system of volume_pd_element_energy.cpp:61-155; Neo-Hookean: implicit function
+// theorem on the proximal optimality, neohookean_pd_element_energy.cpp:133-165).
+template <typename T>
+__device__ void project_diff(int type, T mu, T la, T k, const T* U, const T* sig, const T* V, const T* sp, const T* dF,
+                             T* out) {
     if (type == 0) {
         T R[9], S[9], one[3] = {T(1), T(1), T(1)};
         usvt(U, one, V, R);
@@ -351,8 +360,7 @@ __device__ void project_diff(int type, T mu, T la, T k, const T* U, const T* sig
     T dU[9], dV[9], ds[3];
     dsvd3(U, sig, V, dF, dU, ds, dV);
     if (type == 1) {
-        T D[3];
-        volume_D(sig, D);
+        const T* D = sp;
         const T a0 = sig[0] + D[0], a1 = sig[1] + D[1], a2 = sig[2] + D[2];
         const T g[3] = {a1 * a2, a0 * a2, a0 * a1};
         // H(i,j) = prod over the remaining index (i != j), 0 on the diagonal
@@ -387,8 +395,7 @@ __device__ void project_diff(int type, T mu, T la, T k, const T* U, const T* sig
         for (int i = 0; i < 9; ++i) out[i] = dF[i] + t1[i] + t2[i] + t3[i];
         return;
     }
-    T ss[3];
-    nh_prox(mu, la, k, sig, ss);
+    const T* ss = sp;
     T H[9];
     nh_hessian(mu, la, k, ss, H);
     H[0] += T(1e-9); H[4] += T(1e-9); H[8] += T(1e-9);

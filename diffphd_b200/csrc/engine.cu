@@ -645,6 +645,8 @@ void Engine::build_device(int threads) {
         d_type_k.upload(tk);
         d_off_k.upload(ok);
         d_dmat_dev.alloc(std::max<size_t>(1, npk.size()) * sizeof(double));
+        d_param_work.alloc(param_reduce_words(m) * sizeof(double));
+        CUDA_OK(cudaMemset(d_param_work.p, 0, d_param_work.bytes));
         d_dpar_dev.alloc(std::max(1, off) * sizeof(double));
         d_dstate_dev.alloc(3 * sizeof(double));
         d_adjnorm.alloc(2 * sizeof(double));
@@ -1851,12 +1853,13 @@ void Engine::backward_core(const double* d_q_next, const double* d_gq, const dou
     const double vol_over_s = M.vol / M.s;
     launch_adj_prepare(n3, d_gq, d_gv, 1.0 / h, d_gbar.as<double>(), d_dq, d_part_adj.as<double>(),
                        d_adjnorm.as<double>(), st);
-    d_J.alloc((size_t)m * M.s * 81 * sizeof(double));
+    const size_t samples = ((size_t)m * M.s + 31) / 32 * 32;  // stored by blocks of 32
+    d_J.alloc(samples * 81 * sizeof(double));
     Ctrl* c = d_ctrl.as<Ctrl>();
     init_ctrl(h_ctrl_, 1, o, o.max_pd_iter, o.bwd_clip);
     CUDA_OK(cudaMemcpyAsync(c, h_ctrl_, sizeof(Ctrl), cudaMemcpyHostToDevice, st));
     const bool j32 = o.fp32_bulk && o.bwd_solver == 1;
-    if (j32) d_J32.alloc((size_t)m * M.s * 48 * sizeof(float));
+    if (j32) d_J32.alloc(samples * 48 * sizeof(float));
     launch_jac_build(m, M.k, M.s, dE.as<int>(), d_q_next, dgrad.as<double>(), M.hex, vol_over_s, ep,
                      o.bwd_mean_stiffness, o.bwd_eigen_filter, d_J.as<double>(), j32 ? d_J32.as<float>() : nullptr, c,
                      st);
@@ -1981,7 +1984,8 @@ void Engine::backward_core(const double* d_q_next, const double* d_gq, const dou
     launch_param_grad(m, M.k, M.s, dE.as<int>(), d_q_next, d_x.as<double>(), dgrad.as<double>(), M.hex, vol_over_s,
                       ep, d_gw.as<double>(), d_gmat.as<double>(), d_gnh.as<double>(), st);
     launch_param_reduce(m, ne, d_np_k.as<int>(), d_type_k.as<int>(), d_off_k.as<int>(), d_gw.as<double>(),
-                        d_gmat.as<double>(), d_gnh.as<double>(), d_dmat_w ? d_dmat_w : d_dmat_dev.as<double>(),
+                        d_gmat.as<double>(), d_gnh.as<double>(), d_param_work.as<double>(),
+                        d_dmat_w ? d_dmat_w : d_dmat_dev.as<double>(),
                         d_dparams ? d_dparams : d_dpar_dev.as<double>(), st);
     launches_ += 3;
     CUDA_OK(cudaGetLastError());

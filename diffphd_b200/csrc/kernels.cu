@@ -976,30 +976,54 @@ __device__ void jacobi_eig9(double* A, double* Q) {
     }
 }
 
+// The cached Jacobians are stored by blocks of 32 samples, entry by entry within a block (entry k of sample t at
+// ((t / 32) 81 + k) 32 + t % 32), so that the lanes of a warp -- consecutive samples -- read and write consecutive
+// addresses.  (With a sample's 81 values together, each access of a warp touched 32 lines; entry by entry over all
+// samples, a warp's 81 streams lay megabytes apart.)
+constexpr int kJStride = 32;
+__device__ __forceinline__ size_t j_base(int t, int entries) { return (size_t)(t >> 5) * (entries * 32) + (t & 31); }
+
 // FP32 copy of a symmetric 9x9 Jacobian (the projections' differentials are Hessians of scalar functions):
-// upper triangle, row by row, (J_ic + J_ci) / 2, padded to 48 floats for 16-byte loads.
-constexpr int kJ32Stride = 48;
-__device__ __forceinline__ void pack_sym32(const double* Jt, float* o) {
+// upper triangle, row by row, (J_ic + J_ci) / 2, padded to 48 floats: 12 vectors of 4, blocked like the doubles.
+constexpr int kJ32Vecs = 12;
+__device__ __forceinline__ void pack_sym32(const double* Jt, float4* o) {
+    constexpr int N = kJStride;
+    float buf[4 * kJ32Vecs];
     int k = 0;
+#pragma unroll
     for (int i = 0; i < 9; ++i)
-        for (int c = i; c < 9; ++c) o[k++] = (float)(0.5 * (Jt[c * 9 + i] + Jt[i * 9 + c]));
-    for (; k < kJ32Stride; ++k) o[k] = 0.f;
+#pragma unroll
+        for (int c = i; c < 9; ++c) buf[k++] = (float)(0.5 * (Jt[(c * 9 + i) * N] + Jt[(i * 9 + c) * N]));
+#pragma unroll
+    for (int j = 45; j < 48; ++j) buf[j] = 0.f;
+#pragma unroll
+    for (int j = 0; j < kJ32Vecs; ++j) o[j * N] = make_float4(buf[4 * j], buf[4 * j + 1], buf[4 * j + 2], buf[4 * j + 3]);
 }
 
 template <int K, int S>
-__global__ void __launch_bounds__(128) k_jac_build(int m, const int* __restrict__ E, const double* __restrict__ q,
+__global__ void __launch_bounds__(128, 3) k_jac_build(int m, const int* __restrict__ E, const double* __restrict__ q,
                                                    const double* __restrict__ grad, double vol_over_s, EnergyPack ep,
                                                    int mean_w, int filter, double* __restrict__ J,
-                                                   float* __restrict__ J32, Ctrl* ctrl) {
+                                                   float4* __restrict__ J32, Ctrl* ctrl) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int e = t / S, smp = t % S;
     if (e >= m) return;
+    constexpr int N = kJStride;
     const double* g = (S == 8) ? grad + smp * 24 : grad + (size_t)e * 12;
     double F[9], U[9], V[9], sig[3];
     def_grad<K>(E, e, q, g, F);
     svd3<double>(F, U, sig, V);
-    double* Jt = J + (size_t)t * 81;
-    double wsum = 0;
+    double* Jt = J + j_base(t, 81);
+    double wsum = 0, w_k[kMaxEnergies] = {}, sp[kMaxEnergies][3] = {};
+#pragma unroll 1
+    for (int k = 0; k < ep.count; ++k) {
+        const ElemEnergyDev& en = ep.en[k];
+        if (en.mask && !en.mask[e]) continue;
+        w_k[k] = (mean_w ? en.w_mean : ld_weight<double>(en, e)) * vol_over_s;
+        wsum += w_k[k];
+        project_point<double>(en.type, en.mu, en.la, en.w_mean, sig, sp[k]);
+    }
+#pragma unroll 1
     for (int col = 0; col < 9; ++col) {
         double dF[9];
 #pragma unroll
@@ -1007,21 +1031,20 @@ __global__ void __launch_bounds__(128) k_jac_build(int m, const int* __restrict_
         double out[9];
 #pragma unroll
         for (int i = 0; i < 9; ++i) out[i] = 0.0;
+#pragma unroll 1
         for (int k = 0; k < ep.count; ++k) {
             const ElemEnergyDev& en = ep.en[k];
             if (en.mask && !en.mask[e]) continue;
-            const double w = (mean_w ? en.w_mean : ld_weight<double>(en, e)) * vol_over_s;
-            if (col == 0) wsum += w;
             double d[9];
-            project_diff<double>(en.type, en.mu, en.la, en.w_mean, U, sig, V, dF, d);
+            project_diff<double>(en.type, en.mu, en.la, en.w_mean, U, sig, V, sp[k], dF, d);
 #pragma unroll
-            for (int i = 0; i < 9; ++i) out[i] += w * d[i];
+            for (int i = 0; i < 9; ++i) out[i] += w_k[k] * d[i];
         }
 #pragma unroll
-        for (int i = 0; i < 9; ++i) Jt[col * 9 + i] = out[i];  // column col (column-major 9x9)
+        for (int i = 0; i < 9; ++i) Jt[(col * 9 + i) * N] = out[i];  // column col (column-major 9x9)
     }
     if (filter == 0) {
-        if (J32) pack_sym32(Jt, J32 + (size_t)t * kJ32Stride);
+        if (J32) pack_sym32(Jt, J32 + j_base(t, kJ32Vecs));
         return;
     }
     // State-adaptive filter of the local Hessian H = wsum I - J (the PD energy's per-sample Hessian), with the
@@ -1030,7 +1053,8 @@ __global__ void __launch_bounds__(128) k_jac_build(int m, const int* __restrict_
     // eigenvalues clamped at 0 (filter 1) or replaced by |lambda| (filter 2).
     double H[81];
     for (int i = 0; i < 9; ++i)
-        for (int j = 0; j < 9; ++j) H[i * 9 + j] = (i == j ? wsum : 0.0) - 0.5 * (Jt[j * 9 + i] + Jt[i * 9 + j]);
+        for (int j = 0; j < 9; ++j)
+            H[i * 9 + j] = (i == j ? wsum : 0.0) - 0.5 * (Jt[(j * 9 + i) * N] + Jt[(i * 9 + j) * N]);
     bool dd = true;
     for (int i = 0; i < 9 && dd; ++i) {
         double off = 0;
@@ -1039,7 +1063,7 @@ __global__ void __launch_bounds__(128) k_jac_build(int m, const int* __restrict_
         dd = !(fabs(H[i * 9 + i]) < off + 1e-5);
     }
     if (dd) {
-        if (J32) pack_sym32(Jt, J32 + (size_t)t * kJ32Stride);
+        if (J32) pack_sym32(Jt, J32 + j_base(t, kJ32Vecs));
         return;
     }
     double Q[81];
@@ -1053,10 +1077,10 @@ __global__ void __launch_bounds__(128) k_jac_build(int m, const int* __restrict_
         for (int j = 0; j < 9; ++j) {
             double h = 0;
             for (int k = 0; k < 9; ++k) h += Q[i * 9 + k] * lam[k] * Q[j * 9 + k];
-            Jt[j * 9 + i] = (i == j ? wsum : 0.0) - h;
+            Jt[(j * 9 + i) * N] = (i == j ? wsum : 0.0) - h;
         }
     atomicAdd(&ctrl->arrive[3], 1u);  // number of filtered samples (diagnostic)
-    if (J32) pack_sym32(Jt, J32 + (size_t)t * kJ32Stride);
+    if (J32) pack_sym32(Jt, J32 + j_base(t, kJ32Vecs));
 }
 
 template <int K, int S>
@@ -1075,7 +1099,8 @@ __global__ void __launch_bounds__(kThreads) k_kpd_elem(int m, const int* __restr
         const double* g = (S == 8) ? grad + smp * 24 : grad + (size_t)e * 12;
         double dF[9];
         def_grad<K>(E, e, u, g, dF);
-        const double* Jt = J + (size_t)t * 81;
+        constexpr int N = kJStride;
+        const double* Jt = J + j_base(t, 81);
         double P[9];
 #pragma unroll
         for (int i = 0; i < 9; ++i) P[i] = 0.0;
@@ -1083,7 +1108,7 @@ __global__ void __launch_bounds__(kThreads) k_kpd_elem(int m, const int* __restr
         for (int col = 0; col < 9; ++col) {
             const double f = dF[col];
 #pragma unroll
-            for (int i = 0; i < 9; ++i) P[i] += __ldg(Jt + col * 9 + i) * f;
+            for (int i = 0; i < 9; ++i) P[i] += __ldg(Jt + (col * 9 + i) * N) * f;
         }
 #pragma unroll
         for (int a = 0; a < K; ++a) {
@@ -1120,7 +1145,7 @@ __global__ void __launch_bounds__(kThreads) k_kpd_elem(int m, const int* __restr
 template <int K, int S>
 __global__ void __launch_bounds__(kThreads) k_kpd_elem32(int m, const int* __restrict__ E,
                                                          const double* __restrict__ u, const double* __restrict__ grad,
-                                                         const float* __restrict__ J32, double* __restrict__ out,
+                                                         const float4* __restrict__ J32, double* __restrict__ out,
                                                          const Ctrl* ctrl) {
     pdl_enter();
     if (ctrl->done) return;
@@ -1132,11 +1157,11 @@ __global__ void __launch_bounds__(kThreads) k_kpd_elem32(int m, const int* __res
     for (int a = 0; a < K; ++a) acc[a][0] = acc[a][1] = acc[a][2] = 0.0;
     if (valid) {
         const double* g = (S == 8) ? grad + smp * 24 : grad + (size_t)e * 12;
-        float Mv[kJ32Stride];
-        const float4* src = reinterpret_cast<const float4*>(J32 + (size_t)t * kJ32Stride);
+        float Mv[4 * kJ32Vecs];
+        const float4* src = J32 + j_base(t, kJ32Vecs);
 #pragma unroll
-        for (int k = 0; k < kJ32Stride / 4; ++k) {
-            const float4 x = __ldg(src + k);
+        for (int k = 0; k < kJ32Vecs; ++k) {
+            const float4 x = __ldg(src + k * kJStride);
             Mv[4 * k] = x.x; Mv[4 * k + 1] = x.y; Mv[4 * k + 2] = x.z; Mv[4 * k + 3] = x.w;
         }
         double dFd[9];
@@ -1582,46 +1607,61 @@ __global__ void __launch_bounds__(kThreads) k_adj_route(int n3, const double* __
     }
 }
 
-// One block per energy: fixed-order sums (deterministic).
-__global__ void k_param_reduce(int m, const int* __restrict__ np_k, const int* __restrict__ type_k,
-                               const int* __restrict__ off_k, const double* __restrict__ gw,
-                               const double* __restrict__ gmat, const double* __restrict__ gnh,
-                               double* __restrict__ dmat, double* __restrict__ dpar) {
+// Sums of the per-element gradient terms of each energy (blockIdx.y), kParamElems elements per block; the energy's last
+// block sums the blocks' partials in order.  One block per energy took 126 us over 40,960 elements and 191 us over
+// 65,536.
+constexpr int kParamElems = 1024;
+__global__ void __launch_bounds__(kThreads) k_param_sums(int m, const double* __restrict__ gw,
+                                                         const double* __restrict__ gmat,
+                                                         const double* __restrict__ gnh, double* __restrict__ part,
+                                                         double* __restrict__ tot, unsigned int* __restrict__ arrive) {
     __shared__ double sh[4 * 32];
-    const int k = blockIdx.x;
-    const int npk = np_k[k], type = type_k[k], off = off_k[k];
-    const double* w = gw + (size_t)k * m;
+    const int k = blockIdx.y;
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int e = threadIdx.x; e < m; e += blockDim.x) {
-        acc[0] += gmat[(size_t)k * m + e];
-        acc[1] += w[e];
-        acc[2] += gnh[((size_t)k * m + e) * 2];
-        acc[3] += gnh[((size_t)k * m + e) * 2 + 1];
+    const int e1 = min(m, (int)(blockIdx.x + 1) * kParamElems);
+    for (int e = blockIdx.x * kParamElems + threadIdx.x; e < e1; e += blockDim.x) {
+        const size_t i = (size_t)k * m + e;
+        acc[0] += gmat[i];
+        acc[1] += gw[i];
+        acc[2] += gnh[2 * i];
+        acc[3] += gnh[2 * i + 1];
     }
     block_sum<4>(acc, sh);
-    __shared__ double tot[4];
+    double* pk = part + (size_t)k * gridDim.x * 4;
     if (threadIdx.x == 0)
-        for (int i = 0; i < 4; ++i) tot[i] = acc[i];
-    __syncthreads();
-    if (threadIdx.x == 0) dmat[k] = tot[0];
-    if (type != 2) {
+        for (int i = 0; i < 4; ++i) pk[blockIdx.x * 4 + i] = acc[i];
+    if (!arrive_last(arrive + k)) return;
+    double t[4];
+    sum_partials<4>(pk, gridDim.x, t, sh);
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 4; ++i) tot[4 * k + i] = t[i];
+        arrive[k] = 0;
+    }
+}
+
+// dl_dmat_w and dl_dparams in the parameter layout of each energy (blockIdx.y), from the sums and per-element terms.
+__global__ void __launch_bounds__(kThreads) k_param_out(int m, const int* __restrict__ np_k,
+                                                        const int* __restrict__ type_k, const int* __restrict__ off_k,
+                                                        const double* __restrict__ gw, const double* __restrict__ tot,
+                                                        double* __restrict__ dmat, double* __restrict__ dpar) {
+    const int k = blockIdx.y, e = blockIdx.x * blockDim.x + threadIdx.x;
+    const int npk = np_k[k], off = off_k[k];
+    const double* t = tot + 4 * k;
+    if (e == 0) dmat[k] = t[0];
+    if (type_k[k] != 2) {
         if (npk == 1) {
-            if (threadIdx.x == 0) dpar[off] = tot[1];
-        } else {
-            for (int e = threadIdx.x; e < m; e += blockDim.x) dpar[off + e] = w[e];
+            if (e == 0) dpar[off] = t[1];
+        } else if (e < m) {
+            dpar[off + e] = gw[(size_t)k * m + e];
         }
-    } else {
-        if (npk == 2) {
-            if (threadIdx.x == 0) {
-                dpar[off] = 2 * tot[1] + tot[2];
-                dpar[off + 1] = tot[3];
-            }
-        } else {
-            for (int e = threadIdx.x; e < m; e += blockDim.x) {
-                dpar[off + 2 * e] = 2 * w[e] + tot[2] / m;
-                dpar[off + 2 * e + 1] = tot[3] / m;
-            }
+    } else if (npk == 2) {
+        if (e == 0) {
+            dpar[off] = 2 * t[1] + t[2];
+            dpar[off + 1] = t[3];
         }
+    } else if (e < m) {
+        dpar[off + 2 * e] = 2 * gw[(size_t)k * m + e] + t[2] / m;
+        dpar[off + 2 * e + 1] = t[3] / m;
     }
 }
 
@@ -1755,8 +1795,9 @@ void launch_jac_build(int m, int k, int s, const int* E, const double* q, const 
                       Ctrl* ctrl, cudaStream_t st) {
     (void)k;
     const int grid = blocks_for((long long)m * s, 128);
-    if (hex) k_jac_build<8, 8><<<grid, 128, 0, st>>>(m, E, q, grad, vol_over_s, ep, mean_w, filter, J, J32, ctrl);
-    else k_jac_build<4, 1><<<grid, 128, 0, st>>>(m, E, q, grad, vol_over_s, ep, mean_w, filter, J, J32, ctrl);
+    float4* J4 = reinterpret_cast<float4*>(J32);
+    if (hex) k_jac_build<8, 8><<<grid, 128, 0, st>>>(m, E, q, grad, vol_over_s, ep, mean_w, filter, J, J4, ctrl);
+    else k_jac_build<4, 1><<<grid, 128, 0, st>>>(m, E, q, grad, vol_over_s, ep, mean_w, filter, J, J4, ctrl);
 }
 
 void launch_kpd_elem32(int m, int k, int s, const int* E, const double* u, const double* grad, int hex,
@@ -1764,8 +1805,9 @@ void launch_kpd_elem32(int m, int k, int s, const int* E, const double* u, const
     (void)k;
     int grid, bs;
     even_grid((long long)m * s, kThreads, 1 << 30, &grid, &bs);
-    if (hex) launch_k(k_kpd_elem32<8, 8>, grid, bs, 0, st, m, E, u, grad, J32, elem_out, ctrl);
-    else launch_k(k_kpd_elem32<4, 1>, grid, bs, 0, st, m, E, u, grad, J32, elem_out, ctrl);
+    const float4* J4 = reinterpret_cast<const float4*>(J32);
+    if (hex) launch_k(k_kpd_elem32<8, 8>, grid, bs, 0, st, m, E, u, grad, J4, elem_out, ctrl);
+    else launch_k(k_kpd_elem32<4, 1>, grid, bs, 0, st, m, E, u, grad, J4, elem_out, ctrl);
 }
 
 void launch_kpd_elem(int m, int k, int s, const int* E, const double* u, const double* grad, int hex, const double* J,
@@ -1968,10 +2010,19 @@ void launch_adj_route(int n3, const double* mu, double mu_norm, const double* gb
         arrive);
 }
 
+size_t param_reduce_words(int m) { return (size_t)kMaxEnergies * (4 * ((m + kParamElems - 1) / kParamElems) + 4 + 1); }
+
 void launch_param_reduce(int m, int ne, const int* np_k, const int* type_k, const int* off_k, const double* gw,
-                         const double* gmat, const double* gnh, double* dl_dmat_w, double* dl_dparams,
+                         const double* gmat, const double* gnh, double* work, double* dl_dmat_w, double* dl_dparams,
                          cudaStream_t st) {
-    if (ne > 0) k_param_reduce<<<ne, kThreads, 0, st>>>(m, np_k, type_k, off_k, gw, gmat, gnh, dl_dmat_w, dl_dparams);
+    if (ne <= 0) return;
+    const int nb = (m + kParamElems - 1) / kParamElems;
+    unsigned int* arrive = reinterpret_cast<unsigned int*>(work);  // zero between calls
+    double* tot = work + kMaxEnergies;
+    double* part = tot + 4 * kMaxEnergies;
+    k_param_sums<<<dim3(nb, ne), kThreads, 0, st>>>(m, gw, gmat, gnh, part, tot, arrive);
+    k_param_out<<<dim3((m + kThreads - 1) / kThreads, ne), kThreads, 0, st>>>(m, np_k, type_k, off_k, gw, tot,
+                                                                             dl_dmat_w, dl_dparams);
 }
 
 template <typename T>

@@ -182,7 +182,9 @@ void launch_velocity(int n3, const double* q_next, const double* q, double inv_h
 
 // Adjoint ------------------------------------------------------------------------------------------
 // Per-sample 9x9 local Jacobians J_s = sum_energies w (vol/s) dBp/dF at q_next (optionally eigen-filtered).
-// With J32 set, also an FP32 packed symmetric copy (48 floats per sample) for the mixed-precision adjoint.
+// Stored by blocks of 32 samples (the arrays hold a whole number of blocks): entry col * 9 + i of sample t at
+// ((t / 32) 81 + col * 9 + i) 32 + t % 32.  With J32 set, also an FP32 packed symmetric copy (12 vectors of 4 floats
+// per sample, blocked the same way) for the mixed-precision adjoint.
 void launch_jac_build(int m, int k, int s, const int* E, const double* q, const double* grad, int hex,
                       double vol_over_s, const EnergyPack& ep, int mean_w, int filter, double* J, float* J32,
                       Ctrl* ctrl, cudaStream_t st);
@@ -407,8 +409,10 @@ void launch_adj_route(int n3, const double* mu, double mu_norm, const double* gb
                       double h2m, double mass, int cap, int gravity, double* dl_dq, double* dl_dv, double* dl_df,
                       double* dl_dstate_p, double* part, unsigned int* arrive, cudaStream_t st);
 // per energy: dl_dmat_w[k] = sum_e gmat[k][e]; dl_dparams from gw / gnh in the parameter layout of the energy.
+// `work`: param_reduce_words(m) doubles, zeroed once.
+size_t param_reduce_words(int m);
 void launch_param_reduce(int m, int ne, const int* np_k, const int* type_k, const int* off_k, const double* gw,
-                         const double* gmat, const double* gnh, double* dl_dmat_w, double* dl_dparams,
+                         const double* gmat, const double* gnh, double* work, double* dl_dmat_w, double* dl_dparams,
                          cudaStream_t st);
 
 }  // namespace dphd
