@@ -515,6 +515,10 @@ void Engine::build_device(int threads) {
     plan32_.vals = d_vals32.as<float>();
     plan32_.xpart = d_xpart32.as<float>();
     // the factor stays in L2 across PD iterations when it takes at most about half of it (126 MB on B200)
+    // small meshes: the FP64 loops run as one kernel (rows of one item, chunks and blocks within its limits)
+    const int longest = *std::max_element(rl.begin(), rl.end());
+    small_loop_ = !(M.has_plane && !M.contact_nodes.empty()) && n3 <= kSmallDofs && m * M.s <= kSmallSamples &&
+                  longest <= seg_cols && chunk <= kSmallChunk && small_loop_supported(M.hex);
     plan64_.keep_in_l2 = d_vals64.bytes <= (64ull << 20) ? 1 : 0;
     plan32_.keep_in_l2 = d_vals32.bytes <= (64ull << 20) ? 1 : 0;
     auto fill_units = [&](auto& P, DeviceBuffer& yrow, bool use) {
@@ -1178,6 +1182,41 @@ bool Engine::build_while_graph(int mode, int cap_iters) {
     return ok;
 }
 
+void Engine::run_small_loop(int mode, int cap_iters, cudaStream_t st) {
+    SmallLoop a;
+    a.n = M.n;
+    a.m = M.m;
+    a.E = dE.as<int>();
+    a.qb = d_qb.as<double>();
+    a.elem_dir = d_elem_dir.as<unsigned char>();
+    a.grad = dgrad.as<double>();
+    a.vol_over_s = M.vol / M.s;
+    a.inv_h2m = M.mass() / (graph_dt_ * graph_dt_);
+    a.ep = energy_pack();
+    a.J = d_J.as<double>();
+    a.x = d_x.as<double>();
+    a.elem_out = d_elem_out64.as<double>();
+    a.node_ptr = d_node_ptr.as<int>();
+    a.node_inc = d_node_inc.as<int>();
+    a.rhs = mode == 0 ? d_qt.as<double>() : d_gbar.as<double>();
+    a.fixed_node = d_fixed_node.as<unsigned char>();
+    a.iperm = d_iperm.as<int>();
+    a.v = d_vperm64.as<double>();
+    a.prev = d_prev_pd.as<double>();
+    a.p = plan64_;
+    a.fixed_dof = d_fixed_dof.as<unsigned char>();
+    a.fixed_val = d_fixed_val.as<double>();
+    a.part_gate = d_part_gate.as<double>();
+    a.part_aa = d_part_aa.as<double>();
+    a.part_upd = d_part_upd.as<double>();
+    a.ctrl = d_ctrl.as<Ctrl>();
+    launch_small_loop(a, M.hex, mode == 0 ? 0 : 1, cap_iters, st);
+    CUDA_OK(cudaGetLastError());
+    CUDA_OK(cudaMemcpyAsync(h_ctrl_, d_ctrl.p, sizeof(Ctrl), cudaMemcpyDeviceToHost, st));
+    CUDA_OK(cudaStreamSynchronize(st));
+    launches_ += 1;
+}
+
 void Engine::run_iterations(int mode, const Options& o, cudaStream_t st) {
     Ctrl* c = d_ctrl.as<Ctrl>();
     cudaGraphExec_t& g = graphs_[mode];
@@ -1190,6 +1229,10 @@ void Engine::run_iterations(int mode, const Options& o, cudaStream_t st) {
     if (g && graph_is_while_[mode] && graph_cap_[mode] != cap_iters) {
         cudaGraphExecDestroy(g);
         g = nullptr;
+    }
+    if (use_while && small_loop_ && (mode == 0 || mode == 2)) {
+        run_small_loop(mode, cap_iters, st);
+        return;
     }
     if (!g && use_while) {
         if (build_while_graph(mode, cap_iters)) {

@@ -235,6 +235,8 @@ private:
     void enqueue_bwd_iteration(cudaStream_t st);
     // mode 0 fwd64, 1 fwd mixed, 2 adjoint fixed point, 3 adjoint PCG (FP64 preconditioner), 4 PCG (FP32 precond.)
     void run_iterations(int mode, const Options& o, cudaStream_t st);
+    void run_small_loop(int mode, int cap_iters, cudaStream_t st);
+    bool small_loop_ = false;  // the FP64 fixed-point loops run as one kernel (small_loop.cu)
     void drop_graphs();
     void check_status(const char* where);
     void check_device() const;

@@ -7,6 +7,8 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "anderson.cuh"
+#include "element.cuh"
 #include "kernels.cuh"
 #include "launch.cuh"
 
@@ -77,34 +79,6 @@ __device__ __forceinline__ void sum_partials(const double* part, int nb, double*
         for (int i = 0; i < NV; ++i) out[i] = v[i];
 }
 
-template <typename T>
-__device__ __forceinline__ T ld_weight(const ElemEnergyDev& en, int e);
-template <>
-__device__ __forceinline__ double ld_weight<double>(const ElemEnergyDev& en, int e) {
-    return en.per_element ? __ldg(en.w + e) : en.w_mean;
-}
-template <>
-__device__ __forceinline__ float ld_weight<float>(const ElemEnergyDev& en, int e) {
-    return en.per_element ? __ldg(en.w32 + e) : (float)en.w_mean;
-}
-
-// Deformation gradient F(i,j) = sum_a x_a[i] grad_a[j] over the element's nodes (FP64 accumulation).
-template <int K>
-__device__ __forceinline__ void def_grad(const int* __restrict__ E, int e, const double* __restrict__ x,
-                                         const double* __restrict__ g, double* F) {
-#pragma unroll
-    for (int i = 0; i < 9; ++i) F[i] = 0.0;
-#pragma unroll
-    for (int a = 0; a < K; ++a) {
-        const int node = __ldg(E + (size_t)e * K + a);
-        const double x0 = x[3 * node], x1 = x[3 * node + 1], x2 = x[3 * node + 2];
-        const double g0 = __ldg(g + a * 3), g1 = __ldg(g + a * 3 + 1), g2 = __ldg(g + a * 3 + 2);
-        F[0] += x0 * g0; F[1] += x1 * g0; F[2] += x2 * g0;
-        F[3] += x0 * g1; F[4] += x1 * g1; F[5] += x2 * g1;
-        F[6] += x0 * g2; F[7] += x1 * g2; F[8] += x2 * g2;
-    }
-}
-
 // ------------------------------------------------------------------------------------------------
 // Forward local step (deformable_projective_dynamics_forward.cpp:186-292), one thread per (element, sample);
 // for hexes the 8 samples of an element are 8 consecutive lanes and are summed by a shuffle butterfly.
@@ -120,75 +94,8 @@ __global__ void __launch_bounds__(kThreads) k_elem_fwd(int m, const int* __restr
                                                        EnergyPack ep, double* __restrict__ out, Ctrl* ctrl) {
     pdl_enter();
     if (ctrl->done) return;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int e = t / S, smp = t % S;
-    const bool valid = e < m;
-    double acc[K][3];
-#pragma unroll
-    for (int a = 0; a < K; ++a) acc[a][0] = acc[a][1] = acc[a][2] = 0.0;
-    if (valid) {
-        const double* g = (S == 8) ? grad + smp * 24 : grad + (size_t)e * 12;
-        double Fd[9], Fbd[9];
-        def_grad<K>(E, e, q, g, Fd);
-        if (elem_dir[e]) def_grad<K>(E, e, qb, g, Fbd);
-        else {
-#pragma unroll
-            for (int i = 0; i < 9; ++i) Fbd[i] = 0.0;
-        }
-        T F[9];
-#pragma unroll
-        for (int i = 0; i < 9; ++i) F[i] = (T)Fd[i];
-        T U[9], V[9], sig[3];
-        svd3<T>(F, U, sig, V);
-        double P[9];
-#pragma unroll
-        for (int i = 0; i < 9; ++i) P[i] = 0.0;
-        bool ok = true;
-        for (int k = 0; k < ep.count; ++k) {
-            const ElemEnergyDev& en = ep.en[k];
-            if (en.mask && !en.mask[e]) continue;
-            const double w = ld_weight<double>(en, e) * vol_over_s;
-            T Bp[9];
-            if (sizeof(T) == 8) {
-                ok = project<T>(en.type, (T)en.mu, (T)en.la, (T)en.w_mean, U, sig, V, Bp) && ok;
-#pragma unroll
-                for (int i = 0; i < 9; ++i) P[i] += w * ((double)Bp[i] - Fbd[i]);
-            } else {
-                ok = project_delta<T>(en.type, (T)en.mu, (T)en.la, (T)en.w_mean, U, sig, V, Bp) && ok;
-#pragma unroll
-                for (int i = 0; i < 9; ++i) P[i] += w * ((Fd[i] - Fbd[i]) + (double)Bp[i]);
-            }
-        }
-        if (!ok) atomicOr(&ctrl->status, (int)kStatusSingularF);
-#pragma unroll
-        for (int a = 0; a < K; ++a) {
-            const double g0 = __ldg(g + a * 3), g1 = __ldg(g + a * 3 + 1), g2 = __ldg(g + a * 3 + 2);
-#pragma unroll
-            for (int i = 0; i < 3; ++i) acc[a][i] = P[i] * g0 + P[i + 3] * g1 + P[i + 6] * g2;
-        }
-    }
-    if (S == 8) {
-#pragma unroll
-        for (int o = 4; o > 0; o >>= 1)
-#pragma unroll
-            for (int a = 0; a < K; ++a)
-#pragma unroll
-                for (int i = 0; i < 3; ++i) acc[a][i] += __shfl_xor_sync(0xffffffffu, acc[a][i], o);
-        if (valid) {
-#pragma unroll
-            for (int a = 0; a < K; ++a)
-                if (a == smp) {
-                    double* o = out + ((size_t)e * K + a) * 3;
-                    o[0] = acc[a][0]; o[1] = acc[a][1]; o[2] = acc[a][2];
-                }
-        }
-    } else if (valid) {
-#pragma unroll
-        for (int a = 0; a < K; ++a) {
-            double* o = out + ((size_t)e * K + a) * 3;
-            o[0] = acc[a][0]; o[1] = acc[a][1]; o[2] = acc[a][2];
-        }
-    }
+    elem_fwd_sample<T, K, S>(blockIdx.x * blockDim.x + threadIdx.x, m, E, LdPlain{q}, qb, elem_dir, grad, vol_over_s, ep,
+                             out, &ctrl->status);
 }
 
 // Node gathers run kGatherLanes lanes per node (strided over the node's incident element outputs and its CSR
@@ -683,7 +590,6 @@ __global__ void __launch_bounds__(kThreads) k_spmv_ST_fin(SpmvPlan<T> p, double*
 // `head`.  k_aa_reduce pushes the new entry, forms the Gram system and solves it in the last block;
 // k_aa_update applies the extrapolation, re-imposes Dirichlet values and evaluates the stop rule.
 // ------------------------------------------------------------------------------------------------
-constexpr int kAaVals = 2 * kMaxWindow + 2;  // new Gram column, right-hand side, |g|^2, |x_raw|^2
 
 __global__ void __launch_bounds__(kThreads) k_aa_reduce(int n3, const double* __restrict__ x,
                                                         const double* __restrict__ xr,
@@ -746,92 +652,7 @@ __global__ void __launch_bounds__(kThreads) k_aa_reduce(int n3, const double* __
         return;
     }
     if (m < 1) return;
-    // Extend the stored Gram matrix by the new difference's column, then solve
-    // (dG^T dG + reg I) gamma = dG^T g, reg = max(1e-6 |dG|_F^2 / m, 1e-12), by Cholesky.  All loops run to
-    // kMaxWindow with guards so that the small arrays stay in registers; the stored entries are loaded
-    // independently (one round trip) rather than inside the factorisation.
-    const int snew = (head + m - 1) % W;
-    double A[kMaxWindow][kMaxWindow], b[kMaxWindow];
-#pragma unroll
-    for (int i = 0; i < kMaxWindow; ++i)
-#pragma unroll
-        for (int j = 0; j < kMaxWindow; ++j)
-            if (i < m && j < m)
-                A[i][j] = (i == m - 1) ? tot[j] : (j == m - 1) ? tot[i] : ctrl->gram[(head + i) % W][(head + j) % W];
-#pragma unroll
-    for (int j = 0; j < kMaxWindow; ++j)
-        if (j < m) {
-            const int sj = (head + j) % W;
-            ctrl->gram[snew][sj] = tot[j];
-            ctrl->gram[sj][snew] = tot[j];
-        }
-    double fro = 0;
-#pragma unroll
-    for (int j = 0; j < kMaxWindow; ++j)
-        if (j < m) fro += A[j][j];
-    const double reg = fmax(1e-6 * fro / m, 1e-12);
-#pragma unroll
-    for (int i = 0; i < kMaxWindow; ++i)
-        if (i < m) {
-            A[i][i] += reg;
-            b[i] = tot[kMaxWindow + i];
-        }
-    // one reciprocal per column (a single thread runs this: FP64 divisions dominate its latency)
-    double inv_diag[kMaxWindow];
-#pragma unroll
-    for (int j = 0; j < kMaxWindow; ++j) {
-        inv_diag[j] = 0.0;
-        if (j < m) {
-            double d = A[j][j];
-#pragma unroll
-            for (int k = 0; k < kMaxWindow; ++k)
-                if (k < j) d -= A[j][k] * A[j][k];
-            d = sqrt(fmax(d, 1e-300));
-            A[j][j] = d;
-            const double inv = 1.0 / d;
-            inv_diag[j] = inv;
-#pragma unroll
-            for (int i = 0; i < kMaxWindow; ++i)
-                if (i > j && i < m) {
-                    double t = A[i][j];
-#pragma unroll
-                    for (int k = 0; k < kMaxWindow; ++k)
-                        if (k < j) t -= A[i][k] * A[j][k];
-                    A[i][j] = t * inv;
-                }
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < kMaxWindow; ++i)
-        if (i < m) {
-            double t = b[i];
-#pragma unroll
-            for (int k = 0; k < kMaxWindow; ++k)
-                if (k < i) t -= A[i][k] * b[k];
-            b[i] = t * inv_diag[i];
-        }
-#pragma unroll
-    for (int i = kMaxWindow - 1; i >= 0; --i)
-        if (i < m) {
-            double t = b[i];
-#pragma unroll
-            for (int k = 0; k < kMaxWindow; ++k)
-                if (k > i && k < m) t -= A[k][i] * b[k];
-            b[i] = t * inv_diag[i];
-        }
-    double gn = 0;
-#pragma unroll
-    for (int i = 0; i < kMaxWindow; ++i)
-        if (i < m) gn += b[i] * b[i];
-    gn = sqrt(gn);
-    if (!(gn < 10.0)) {
-        ctrl->restart = 1;
-    } else {
-        ctrl->accept = 1;
-#pragma unroll
-        for (int i = 0; i < kMaxWindow; ++i)
-            if (i < m) ctrl->gamma[i] = b[i];
-    }
+    aa_solve(tot, m, head, W, ctrl->gram, ctrl->gamma, &ctrl->accept, &ctrl->restart);
 }
 
 __global__ void __launch_bounds__(kThreads) k_aa_update(int n3, double* __restrict__ x, const double* __restrict__ xr,
@@ -976,13 +797,6 @@ __device__ void jacobi_eig9(double* A, double* Q) {
     }
 }
 
-// The cached Jacobians are stored by blocks of 32 samples, entry by entry within a block (entry k of sample t at
-// ((t / 32) 81 + k) 32 + t % 32), so that the lanes of a warp -- consecutive samples -- read and write consecutive
-// addresses.  (With a sample's 81 values together, each access of a warp touched 32 lines; entry by entry over all
-// samples, a warp's 81 streams lay megabytes apart.)
-constexpr int kJStride = 32;
-__device__ __forceinline__ size_t j_base(int t, int entries) { return (size_t)(t >> 5) * (entries * 32) + (t & 31); }
-
 // FP32 copy of a symmetric 9x9 Jacobian (the projections' differentials are Hessians of scalar functions):
 // upper triangle, row by row, (J_ic + J_ci) / 2, padded to 48 floats: 12 vectors of 4, blocked like the doubles.
 constexpr int kJ32Vecs = 12;
@@ -1011,7 +825,7 @@ __global__ void __launch_bounds__(128, 3) k_jac_build(int m, const int* __restri
     constexpr int N = kJStride;
     const double* g = (S == 8) ? grad + smp * 24 : grad + (size_t)e * 12;
     double F[9], U[9], V[9], sig[3];
-    def_grad<K>(E, e, q, g, F);
+    def_grad<K>(E, e, LdPlain{q}, g, F);
     svd3<double>(F, U, sig, V);
     double* Jt = J + j_base(t, 81);
     double wsum = 0, w_k[kMaxEnergies] = {}, sp[kMaxEnergies][3] = {};
@@ -1089,56 +903,7 @@ __global__ void __launch_bounds__(kThreads) k_kpd_elem(int m, const int* __restr
                                                        double* __restrict__ out, const Ctrl* ctrl) {
     pdl_enter();
     if (ctrl->done) return;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int e = t / S, smp = t % S;
-    const bool valid = e < m;
-    double acc[K][3];
-#pragma unroll
-    for (int a = 0; a < K; ++a) acc[a][0] = acc[a][1] = acc[a][2] = 0.0;
-    if (valid) {
-        const double* g = (S == 8) ? grad + smp * 24 : grad + (size_t)e * 12;
-        double dF[9];
-        def_grad<K>(E, e, u, g, dF);
-        constexpr int N = kJStride;
-        const double* Jt = J + j_base(t, 81);
-        double P[9];
-#pragma unroll
-        for (int i = 0; i < 9; ++i) P[i] = 0.0;
-#pragma unroll
-        for (int col = 0; col < 9; ++col) {
-            const double f = dF[col];
-#pragma unroll
-            for (int i = 0; i < 9; ++i) P[i] += __ldg(Jt + (col * 9 + i) * N) * f;
-        }
-#pragma unroll
-        for (int a = 0; a < K; ++a) {
-            const double g0 = __ldg(g + a * 3), g1 = __ldg(g + a * 3 + 1), g2 = __ldg(g + a * 3 + 2);
-#pragma unroll
-            for (int i = 0; i < 3; ++i) acc[a][i] = P[i] * g0 + P[i + 3] * g1 + P[i + 6] * g2;
-        }
-    }
-    if (S == 8) {
-#pragma unroll
-        for (int o = 4; o > 0; o >>= 1)
-#pragma unroll
-            for (int a = 0; a < K; ++a)
-#pragma unroll
-                for (int i = 0; i < 3; ++i) acc[a][i] += __shfl_xor_sync(0xffffffffu, acc[a][i], o);
-        if (valid) {
-#pragma unroll
-            for (int a = 0; a < K; ++a)
-                if (a == smp) {
-                    double* o = out + ((size_t)e * K + a) * 3;
-                    o[0] = acc[a][0]; o[1] = acc[a][1]; o[2] = acc[a][2];
-                }
-        }
-    } else if (valid) {
-#pragma unroll
-        for (int a = 0; a < K; ++a) {
-            double* o = out + ((size_t)e * K + a) * 3;
-            o[0] = acc[a][0]; o[1] = acc[a][1]; o[2] = acc[a][2];
-        }
-    }
+    kpd_sample<K, S>(blockIdx.x * blockDim.x + threadIdx.x, m, E, LdPlain{u}, grad, J, out);
 }
 
 // K_pd u from the FP32 packed symmetric Jacobians (mixed precision): P = J dF in FP32, element sums in FP64.
@@ -1165,7 +930,7 @@ __global__ void __launch_bounds__(kThreads) k_kpd_elem32(int m, const int* __res
             Mv[4 * k] = x.x; Mv[4 * k + 1] = x.y; Mv[4 * k + 2] = x.z; Mv[4 * k + 3] = x.w;
         }
         double dFd[9];
-        def_grad<K>(E, e, u, g, dFd);
+        def_grad<K>(E, e, LdPlain{u}, g, dFd);
         float dF[9];
 #pragma unroll
         for (int i = 0; i < 9; ++i) dF[i] = (float)dFd[i];
@@ -1188,20 +953,11 @@ __global__ void __launch_bounds__(kThreads) k_kpd_elem32(int m, const int* __res
                 acc[a][i] = (double)P[i] * g0 + (double)P[i + 3] * g1 + (double)P[i + 6] * g2;
         }
     }
-    if (S == 8) {
-#pragma unroll
-        for (int o = 4; o > 0; o >>= 1)
-#pragma unroll
-            for (int a = 0; a < K; ++a)
-#pragma unroll
-                for (int i = 0; i < 3; ++i) acc[a][i] += __shfl_xor_sync(0xffffffffu, acc[a][i], o);
+    if constexpr (S == 8) {
+        sum_samples(acc, smp);
         if (valid) {
-#pragma unroll
-            for (int a = 0; a < K; ++a)
-                if (a == smp) {
-                    double* o = out + ((size_t)e * K + a) * 3;
-                    o[0] = acc[a][0]; o[1] = acc[a][1]; o[2] = acc[a][2];
-                }
+            double* o = out + ((size_t)e * K + smp) * 3;
+            o[0] = acc[0][0]; o[1] = acc[0][1]; o[2] = acc[0][2];
         }
     } else if (valid) {
 #pragma unroll
@@ -1279,11 +1035,11 @@ __global__ void __launch_bounds__(128) k_param_grad(int m, const int* __restrict
     if (valid) {
         const double* g = (S == 8) ? grad + smp * 24 : grad + (size_t)e * 12;
         double F[9], U[9], V[9], sig[3];
-        def_grad<K>(E, e, q, g, F);
+        def_grad<K>(E, e, LdPlain{q}, g, F);
         svd3<double>(F, U, sig, V);
         // G(i,j) = sum_a mu_a[i] grad_a[j]: then mu_e^T A_s^T M = <G, M>
         double G[9];
-        def_grad<K>(E, e, mu, g, G);
+        def_grad<K>(E, e, LdPlain{mu}, g, G);
         for (int k = 0; k < ep.count && k < kMaxEnergies; ++k) {
             const ElemEnergyDev& en = ep.en[k];
             if (en.mask && !en.mask[e]) continue;

@@ -167,6 +167,43 @@ void launch_sts_cg(const SpmvPlan<T>& p, const T* v, double* z, const double* r,
                    int mu_blocks, Ctrl* ctrl, cudaStream_t st);
 
 
+// The FP64 fixed-point loops of small meshes in one kernel (small_loop.cu): mode 0 the forward loop (rhs = q_tilde), 1 the
+// adjoint (rhs = g_bar, J the cached Jacobians).
+struct SmallLoop {
+    int n = 0, m = 0;
+    const int* E = nullptr;
+    const double* qb = nullptr;
+    const unsigned char* elem_dir = nullptr;
+    const double* grad = nullptr;
+    double vol_over_s = 0, inv_h2m = 0;
+    EnergyPack ep;
+    const double* J = nullptr;
+    double* x = nullptr;
+    double* elem_out = nullptr;
+    const int* node_ptr = nullptr;
+    const int* node_inc = nullptr;
+    const double* rhs = nullptr;
+    const unsigned char* fixed_node = nullptr;
+    const int* iperm = nullptr;
+    double* v = nullptr;
+    double* prev = nullptr;
+    SpmvPlan<double> p;
+    const unsigned char* fixed_dof = nullptr;
+    const double* fixed_val = nullptr;
+    double* part_gate = nullptr;
+    double* part_aa = nullptr;
+    double* part_upd = nullptr;
+    Ctrl* ctrl = nullptr;
+};
+// The rule of this path: us per iteration, launched loop -> one kernel, forward | adjoint:
+//   63 nodes 43 -> 31 | 41 -> 25     425 nodes 49 -> 40 | 44 -> 23     714 nodes (3,840 samples) 51 -> 47 | 41 -> 28
+//   800 nodes (2,835 tets) 55 -> 53 | 43 -> 29     1,053 nodes 57 -> 61 | 44 -> 37: 16 SMs no longer suffice
+constexpr int kSmallChunk = 64;       // largest S^T chunk
+constexpr int kSmallDofs = 10 * 256;  // one degree of freedom per thread of the Anderson blocks, at most 16 of them
+constexpr int kSmallSamples = 4096;
+bool small_loop_supported(bool hex);
+void launch_small_loop(const SmallLoop& a, bool hex, int mode, int cap, cudaStream_t st);
+
 // Anderson acceleration + gate ------------------------------------------------------------------
 void launch_aa_reduce(int n3, const double* x, const double* x_raw, const unsigned char* fixed_dof,
                       const double* fixed_val, double* dG, double* dX, double* last_g, double* last_x, int ld,
