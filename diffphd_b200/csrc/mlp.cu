@@ -63,35 +63,74 @@ __device__ __forceinline__ uint32_t pair16(__nv_bfloat16 lo, __nv_bfloat16 hi) {
     return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
 }
 
+// Shared-memory tiles of 128 BF16 columns: the eight-column chunk c of row r is stored at chunk c ^ (r & 7), so that the
+// fragment loads below (the same chunk of eight consecutive rows, 256 bytes apart) touch all banks instead of four.
+__device__ __forceinline__ int swz(int row, int col) { return row * 128 + (((col >> 3) ^ (row & 7)) << 3) + (col & 7); }
+
+// Four (two) 8x8 BF16 matrices; `p`: this lane's 16-byte row (lanes 8 i .. 8 i + 7: the rows of matrix i).  Lane (g, t)
+// receives elements (g, 2t), (g, 2t + 1) of each, or with trans (2t, g), (2t + 1, g).
+__device__ __forceinline__ void ldsm4(const __nv_bfloat16* p, uint32_t* r) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(p))
+                 : "memory");
+}
+__device__ __forceinline__ void ldsm4t(const __nv_bfloat16* p, uint32_t* r) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(p))
+                 : "memory");
+}
+__device__ __forceinline__ void ldsm2t(const __nv_bfloat16* p, uint32_t* r) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];"
+                 : "=r"(r[0]), "=r"(r[1])
+                 : "r"((uint32_t)__cvta_generic_to_shared(p))
+                 : "memory");
+}
+
 __device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
 __device__ __forceinline__ float gelu_d(float x) {
     return 0.5f * (1.0f + erff(x * 0.70710678118654752f)) + x * 0.3989422804014327f * expf(-0.5f * x * x);
 }
 
 struct Smem {
-    __nv_bfloat16 W1T[kHid * kIn];
-    __nv_bfloat16 W2T[kHid * kHid];
-    __nv_bfloat16 W3T[kOut * kHid];
+    __align__(16) __nv_bfloat16 W1T[kHid * kIn];
+    __align__(16) __nv_bfloat16 W2T[kHid * kHid];  // swizzled
+    __align__(16) __nv_bfloat16 W3T[kOut * kHid];  // swizzled
     float b1[kHid], b2[kHid], b3[kOut];
 };
 struct SmemTrain {
     Smem f;
-    __nv_bfloat16 W2b[kHid * kHid];
-    __nv_bfloat16 W3b[kHid * 16];
-    // staged CTA rows for the weight gradients
-    __nv_bfloat16 x[kRowsPerCta * kIn];
-    __nv_bfloat16 a1[kRowsPerCta * kHid];
-    __nv_bfloat16 a2[kRowsPerCta * kHid];
-    __nv_bfloat16 dz1[kRowsPerCta * kHid];
-    __nv_bfloat16 dz2[kRowsPerCta * kHid];
-    __nv_bfloat16 dz3[kRowsPerCta * 16];
+    __align__(16) __nv_bfloat16 W2b[kHid * kHid];  // swizzled
+    __align__(16) __nv_bfloat16 W3b[kHid * 16];
+    // staged CTA rows for the weight gradients (128-column tiles swizzled)
+    __align__(16) __nv_bfloat16 x[kRowsPerCta * kIn];
+    __align__(16) __nv_bfloat16 a1[kRowsPerCta * kHid];
+    __align__(16) __nv_bfloat16 a2[kRowsPerCta * kHid];
+    __align__(16) __nv_bfloat16 dz1[kRowsPerCta * kHid];
+    __align__(16) __nv_bfloat16 dz2[kRowsPerCta * kHid];
+    __align__(16) __nv_bfloat16 dz3[kRowsPerCta * 16];
     float red[8][kHid * 2 + kOut + 1];
 };
 
+// Eight BF16 of the packed weights: one load where they lie on a 16-byte boundary (the caller's array may not).
+__device__ __forceinline__ uint4 load8(const __nv_bfloat16* src) {
+    if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) return *reinterpret_cast<const uint4*>(src);
+    return make_uint4(pair16(src[0], src[1]), pair16(src[2], src[3]), pair16(src[4], src[5]), pair16(src[6], src[7]));
+}
+// `rows` x 128 BF16 into a swizzled tile, and `count` of them as they are.
+__device__ __forceinline__ void copy_swz(__nv_bfloat16* dst, const __nv_bfloat16* src, int rows) {
+    for (int i = threadIdx.x; i < rows * 16; i += blockDim.x)
+        *reinterpret_cast<uint4*>(dst + swz(i >> 4, (i & 15) * 8)) = load8(src + 8 * i);
+}
+__device__ __forceinline__ void copy_plain(__nv_bfloat16* dst, const __nv_bfloat16* src, int count) {
+    for (int i = threadIdx.x; i < count / 8; i += blockDim.x) *reinterpret_cast<uint4*>(dst + 8 * i) = load8(src + 8 * i);
+}
+
 __device__ void load_weights(Smem& s, const MlpParams& p) {
-    for (int i = threadIdx.x; i < kHid * kIn; i += blockDim.x) s.W1T[i] = p.W1T[i];
-    for (int i = threadIdx.x; i < kHid * kHid; i += blockDim.x) s.W2T[i] = p.W2T[i];
-    for (int i = threadIdx.x; i < kOut * kHid; i += blockDim.x) s.W3T[i] = p.W3T[i];
+    copy_plain(s.W1T, p.W1T, kHid * kIn);
+    copy_swz(s.W2T, p.W2T, kHid);
+    copy_swz(s.W3T, p.W3T, kOut);
     for (int i = threadIdx.x; i < kHid; i += blockDim.x) {
         s.b1[i] = p.b1[i];
         s.b2[i] = p.b2[i];
@@ -134,35 +173,43 @@ __device__ __forceinline__ void to_afrag(float (*c)[4], uint32_t (*a)[4]) {
     }
 }
 
-// C (16 x 128) = A (16 x 128, 8 k-steps) * B, B from [n][k] storage with row stride 128, plus bias.
+// C (16 x 128) = A (16 x 128, 8 k-steps) * B, B from swizzled [n][k] storage, plus bias.  The k-steps are the outer loop:
+// the sixteen accumulators are independent, and each still adds its k-steps in order.
 __device__ __forceinline__ void layer_hh(const __nv_bfloat16* BT, const float* bias, uint32_t (*a)[4],
                                          float (*c)[4]) {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int lane = threadIdx.x & 31, t = lane & 3;
+    const int mat = lane >> 3, mr = lane & 7;
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
         c[j][0] = bias ? bias[8 * j + 2 * t] : 0.f;
         c[j][1] = bias ? bias[8 * j + 2 * t + 1] : 0.f;
         c[j][2] = c[j][0];
         c[j][3] = c[j][1];
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-            const uint32_t b[2] = {ld32(&BT[(8 * j + g) * kHid + 16 * kk + 2 * t]),
-                                   ld32(&BT[(8 * j + g) * kHid + 16 * kk + 2 * t + 8])};
-            mma16816(c[j], a[kk], b);
-        }
     }
+#pragma unroll
+    for (int kk = 0; kk < 8; kk += 2)
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            uint32_t b[4];  // two k-steps
+            ldsm4(BT + swz(8 * j + mr, 16 * kk + 8 * mat), b);
+            mma16816(c[j], a[kk], b);
+            mma16816(c[j], a[kk + 1], b + 2);
+        }
 }
 
 __device__ __forceinline__ void layer3(const Smem& s, uint32_t (*a)[4], float* c) {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int lane = threadIdx.x & 31, t = lane & 3;
+    const int mat = lane >> 3, mr = lane & 7;
     c[0] = s.b3[2 * t];
     c[1] = s.b3[2 * t + 1];
     c[2] = c[0];
     c[3] = c[1];
 #pragma unroll
-    for (int kk = 0; kk < 8; ++kk) {
-        const uint32_t b[2] = {ld32(&s.W3T[g * kHid + 16 * kk + 2 * t]), ld32(&s.W3T[g * kHid + 16 * kk + 2 * t + 8])};
+    for (int kk = 0; kk < 8; kk += 2) {
+        uint32_t b[4];
+        ldsm4(s.W3T + swz(mr, 16 * kk + 8 * mat), b);
         mma16816(c, a[kk], b);
+        mma16816(c, a[kk + 1], b + 2);
     }
 }
 
@@ -216,33 +263,41 @@ __global__ void __launch_bounds__(256) k_mlp_train(MlpParams p, const __nv_bfloa
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SmemTrain& s = *reinterpret_cast<SmemTrain*>(smem_raw);
     load_weights(s.f, p);
-    for (int i = threadIdx.x; i < kHid * kHid; i += blockDim.x) s.W2b[i] = p.W2b[i];
-    for (int i = threadIdx.x; i < kHid * 16; i += blockDim.x) s.W3b[i] = p.W3b[i];
+    copy_swz(s.W2b, p.W2b, kHid);
+    copy_plain(s.W3b, p.W3b, kHid * 16);
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int rl = warp * 16;  // local row base
     const int r0 = blockIdx.x * kRowsPerCta + rl;
     // Rows of the warp's tiles are staged in shared memory as soon as they are final (A-fragment order back
     // to row-major), so that only the packed GELU derivatives stay live across the backward pass.
-    auto stage = [&](__nv_bfloat16* dst, int ld, const uint32_t (*fr)[4], int ksteps) {
-        for (int kk = 0; kk < ksteps; ++kk) {
-            *reinterpret_cast<uint32_t*>(&dst[(rl + g) * ld + 16 * kk + 2 * t]) = fr[kk][0];
-            *reinterpret_cast<uint32_t*>(&dst[(rl + g + 8) * ld + 16 * kk + 2 * t]) = fr[kk][1];
-            *reinterpret_cast<uint32_t*>(&dst[(rl + g) * ld + 16 * kk + 2 * t + 8]) = fr[kk][2];
-            *reinterpret_cast<uint32_t*>(&dst[(rl + g + 8) * ld + 16 * kk + 2 * t + 8]) = fr[kk][3];
+    auto put = [&](__nv_bfloat16* at, uint32_t v) { *reinterpret_cast<uint32_t*>(at) = v; };
+    auto stage = [&](__nv_bfloat16* dst, const uint32_t (*fr)[4]) {  // 128 columns
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk) {
+            put(dst + swz(rl + g, 16 * kk + 2 * t), fr[kk][0]);
+            put(dst + swz(rl + g + 8, 16 * kk + 2 * t), fr[kk][1]);
+            put(dst + swz(rl + g, 16 * kk + 2 * t + 8), fr[kk][2]);
+            put(dst + swz(rl + g + 8, 16 * kk + 2 * t + 8), fr[kk][3]);
         }
+    };
+    auto stage16 = [&](__nv_bfloat16* dst, const uint32_t* fr) {  // 16 columns
+        put(dst + (rl + g) * 16 + 2 * t, fr[0]);
+        put(dst + (rl + g + 8) * 16 + 2 * t, fr[1]);
+        put(dst + (rl + g) * 16 + 2 * t + 8, fr[2]);
+        put(dst + (rl + g + 8) * 16 + 2 * t + 8, fr[3]);
     };
     // ---- forward ----
     uint32_t ax[1][4];
     load_x(X, r0, n, ax[0]);
-    stage(s.x, kIn, ax, 1);
+    stage16(s.x, ax[0]);
     float c[16][4];
     layer1(s.f, ax[0], c);  // z1
     // gelu'(z1) and gelu'(z2) are parked (BF16, accumulator order) in the dz1 / dz2 tiles, which each thread
     // later overwrites at the same positions with its own dz values
     auto park = [&](__nv_bfloat16* dst, int j, uint32_t lo, uint32_t hi) {
-        *reinterpret_cast<uint32_t*>(&dst[(rl + g) * kHid + 8 * j + 2 * t]) = lo;
-        *reinterpret_cast<uint32_t*>(&dst[(rl + g + 8) * kHid + 8 * j + 2 * t]) = hi;
+        put(dst + swz(rl + g, 8 * j + 2 * t), lo);
+        put(dst + swz(rl + g + 8, 8 * j + 2 * t), hi);
     };
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
@@ -252,7 +307,7 @@ __global__ void __launch_bounds__(256) k_mlp_train(MlpParams p, const __nv_bfloa
     }
     uint32_t af[8][4];
     to_afrag(c, af);  // a1
-    stage(s.a1, kHid, af, 8);
+    stage(s.a1, af);
     layer_hh(s.f.W2T, s.f.b2, af, c);  // z2
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
@@ -261,7 +316,7 @@ __global__ void __launch_bounds__(256) k_mlp_train(MlpParams p, const __nv_bfloa
         for (int e = 0; e < 4; ++e) c[j][e] = gelu(c[j][e]);
     }
     to_afrag(c, af);  // a2
-    stage(s.a2, kHid, af, 8);
+    stage(s.a2, af);
     float o[4];
     layer3(s.f, af, o);
     // ---- loss gradient dz3 = 2 (pred - y) / n (3 used outputs), and the loss ----
@@ -278,7 +333,7 @@ __global__ void __launch_bounds__(256) k_mlp_train(MlpParams p, const __nv_bfloa
     }
     // ---- backward ----
     const uint32_t adz3[1][4] = {{pack_bf16(dz3[0], dz3[1]), pack_bf16(dz3[2], dz3[3]), 0u, 0u}};
-    stage(s.dz3, 16, adz3, 1);
+    stage16(s.dz3, adz3[0]);
     float bs[2];
     colsum(dz3, bs[0], bs[1]);
     if (lane < 4) {
@@ -290,9 +345,10 @@ __global__ void __launch_bounds__(256) k_mlp_train(MlpParams p, const __nv_bfloa
     for (int of = 16; of > 0; of >>= 1) ls += __shfl_xor_sync(0xffffffffu, ls, of);
     if (lane == 0) s.red[warp][2 * kHid + kOut] = ls;
     auto unpack_mul = [&](float* cj, const __nv_bfloat16* src, int j) {
-        const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&src[(rl + g) * kHid + 8 * j + 2 * t]));
+        const float2 lo =
+            __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(src + swz(rl + g, 8 * j + 2 * t)));
         const float2 hi =
-            __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&src[(rl + g + 8) * kHid + 8 * j + 2 * t]));
+            __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(src + swz(rl + g + 8, 8 * j + 2 * t)));
         cj[0] *= lo.x;
         cj[1] *= lo.y;
         cj[2] *= hi.x;
@@ -312,7 +368,7 @@ __global__ void __launch_bounds__(256) k_mlp_train(MlpParams p, const __nv_bfloa
         }
     }
     to_afrag(c, af);  // dz2
-    stage(s.dz2, kHid, af, 8);
+    stage(s.dz2, af);
     // da1 = dz2 W2^T, B from W2b ([in][out]); dz1 = da1 * gelu'(z1)
     layer_hh(s.W2b, nullptr, af, c);
 #pragma unroll
@@ -325,7 +381,7 @@ __global__ void __launch_bounds__(256) k_mlp_train(MlpParams p, const __nv_bfloa
         }
     }
     to_afrag(c, af);  // dz1
-    stage(s.dz1, kHid, af, 8);
+    stage(s.dz1, af);
     __syncthreads();
     float* P = part + (size_t)blockIdx.x * kPartSize;
     // biases and loss (fixed warp order)
@@ -338,84 +394,127 @@ __global__ void __launch_bounds__(256) k_mlp_train(MlpParams p, const __nv_bfloa
         else P[kPartLoss] = v;
     }
     // ---- weight gradients over the CTA's 128 rows: D[m][n] = sum_r L[r][m] R[r][n] ----
-    // A[m][k] = L[k][m] (transposed tile), B[k][n] = R[k][n].
-    auto wgrad = [&](const __nv_bfloat16* L, int ldl, int m0, const __nv_bfloat16* R, int ldr, int n0, float* acc) {
-        acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
-        for (int kk = 0; kk < kRowsPerCta / 16; ++kk) {
-            const int k0 = 16 * kk;
-            uint32_t a[4], b[2];
-            a[0] = pair16(L[(k0 + 2 * t) * ldl + m0 + g], L[(k0 + 2 * t + 1) * ldl + m0 + g]);
-            a[1] = pair16(L[(k0 + 2 * t) * ldl + m0 + g + 8], L[(k0 + 2 * t + 1) * ldl + m0 + g + 8]);
-            a[2] = pair16(L[(k0 + 2 * t + 8) * ldl + m0 + g], L[(k0 + 2 * t + 9) * ldl + m0 + g]);
-            a[3] = pair16(L[(k0 + 2 * t + 8) * ldl + m0 + g + 8], L[(k0 + 2 * t + 9) * ldl + m0 + g + 8]);
-            b[0] = pair16(R[(k0 + 2 * t) * ldr + n0 + g], R[(k0 + 2 * t + 1) * ldr + n0 + g]);
-            b[1] = pair16(R[(k0 + 2 * t + 8) * ldr + n0 + g], R[(k0 + 2 * t + 9) * ldr + n0 + g]);
-            mma16816(acc, a, b);
-        }
-    };
+    // A[m][k] = L[k][m] and B[k][n] = R[k][n] are both transposed loads of row-major tiles; a warp keeps the fragments of
+    // its 16 rows of A over all its column tiles.
+    constexpr int kSteps = kRowsPerCta / 16;
+    const int mat = lane >> 3, mr = lane & 7;
     auto store = [&](float* dst, int ld, int m0, int n0, const float* acc) {
         dst[(m0 + g) * ld + n0 + 2 * t] = acc[0];
         dst[(m0 + g) * ld + n0 + 2 * t + 1] = acc[1];
         dst[(m0 + g + 8) * ld + n0 + 2 * t] = acc[2];
         dst[(m0 + g + 8) * ld + n0 + 2 * t + 1] = acc[3];
     };
+    uint32_t A[kSteps][4];
     // dW2 [in][out] = a1^T dz2: warp owns input rows [16w, 16w+16)
-    for (int j = 0; j < 16; ++j) {
-        float acc[4];
-        wgrad(s.a1, kHid, 16 * warp, s.dz2, kHid, 8 * j, acc);
-        store(P + kPartW2, kHid, 16 * warp, 8 * j, acc);
-    }
-    // dW1 [in=16][out] = x^T dz1: warp owns output n-tiles 2w, 2w+1
-    for (int jj = 0; jj < 2; ++jj) {
-        float acc[4];
-        wgrad(s.x, kIn, 0, s.dz1, kHid, 8 * (2 * warp + jj), acc);
-        store(P + kPartW1, kHid, 0, 8 * (2 * warp + jj), acc);
+#pragma unroll
+    for (int kk = 0; kk < kSteps; ++kk)
+        ldsm4t(s.a1 + swz(16 * kk + (mat >> 1) * 8 + mr, 16 * warp + (mat & 1) * 8), A[kk]);
+#pragma unroll 2
+    for (int j = 0; j < 16; j += 2) {
+        float acc[2][4] = {};
+#pragma unroll
+        for (int kk = 0; kk < kSteps; ++kk) {
+            uint32_t B[4];  // two n-tiles
+            ldsm4t(s.dz2 + swz(16 * kk + (mat & 1) * 8 + mr, 8 * (j + (mat >> 1))), B);
+            mma16816(acc[0], A[kk], B);
+            mma16816(acc[1], A[kk], B + 2);
+        }
+        store(P + kPartW2, kHid, 16 * warp, 8 * j, acc[0]);
+        store(P + kPartW2, kHid, 16 * warp, 8 * (j + 1), acc[1]);
     }
     // dW3 [hidden][out=8] = a2^T dz3: warp owns hidden rows [16w, 16w+16)
     {
-        float acc[4];
-        wgrad(s.a2, kHid, 16 * warp, s.dz3, 16, 0, acc);
+        float acc[4] = {};
+#pragma unroll
+        for (int kk = 0; kk < kSteps; ++kk) {
+            uint32_t B[2];
+            ldsm4t(s.a2 + swz(16 * kk + (mat >> 1) * 8 + mr, 16 * warp + (mat & 1) * 8), A[kk]);
+            ldsm2t(s.dz3 + (16 * kk + (mat & 1) * 8 + mr) * 16, B);
+            mma16816(acc, A[kk], B);
+        }
         store(P + kPartW3, kOut, 16 * warp, 0, acc);
+    }
+    // dW1 [in=16][out] = x^T dz1: warp owns output n-tiles 2w, 2w+1
+    {
+        float acc[2][4] = {};
+#pragma unroll
+        for (int kk = 0; kk < kSteps; ++kk) {
+            uint32_t B[4];
+            ldsm4t(s.x + (16 * kk + (mat >> 1) * 8 + mr) * 16 + (mat & 1) * 8, A[kk]);
+            ldsm4t(s.dz1 + swz(16 * kk + (mat & 1) * 8 + mr, 8 * (2 * warp + (mat >> 1))), B);
+            mma16816(acc[0], A[kk], B);
+            mma16816(acc[1], A[kk], B + 2);
+        }
+        store(P + kPartW1, kHid, 0, 8 * (2 * warp), acc[0]);
+        store(P + kPartW1, kHid, 0, 8 * (2 * warp + 1), acc[1]);
     }
 }
 
-// Sum of the CTA partials (fixed order), AdamW on the FP32 masters, BF16 re-pack; one thread per parameter.
-__global__ void k_mlp_adamw(MlpParams p, const float* __restrict__ part, int nblocks, float lr, float beta1,
-                            float beta2, float eps, float wd, int step, float* __restrict__ m, float* __restrict__ v,
-                            float* __restrict__ grad_out, float* __restrict__ loss_out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0 && loss_out) {
+// Sum of the CTA partials, AdamW on the FP32 masters, BF16 re-pack: a block takes 32 consecutive parameters and its eight
+// warps an eighth of the partials each (in order; the eight sums are added in warp order).  One thread per parameter over
+// all partials took 44 us for 512 of them (42 MB): 78 blocks with a serial chain of additions.
+constexpr int kAdamWarps = 8;
+__global__ void __launch_bounds__(32 * kAdamWarps) k_mlp_adamw(MlpParams p, const float* __restrict__ part, int nblocks,
+                                                               float lr, float beta1, float beta2, float eps, float wd,
+                                                               int step, float* __restrict__ m, float* __restrict__ v,
+                                                               float* __restrict__ grad_out,
+                                                               float* __restrict__ loss_out) {
+    __shared__ float sums[kAdamWarps][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + lane;
+    if (blockIdx.x == gridDim.x - 1) {  // the loss: one running sum over the partials in order
+        if (w != 0 || !loss_out) return;
         float l = 0.f;
-        for (int b = 0; b < nblocks; ++b) l += part[(size_t)b * kPartSize + kPartLoss];
-        *loss_out = l;
+        for (int b = 0; b < nblocks; b += 32) {
+            const float t = b + lane < nblocks ? part[(size_t)(b + lane) * kPartSize + kPartLoss] : 0.f;
+            for (int u = 0; u < min(32, nblocks - b); ++u) l += __shfl_sync(0xffffffffu, t, u);
+        }
+        if (lane == 0) *loss_out = l;
+        return;
     }
-    if (i >= kPartLoss) return;
+    const int b0 = (int)((long long)nblocks * w / kAdamWarps), b1 = (int)((long long)nblocks * (w + 1) / kAdamWarps);
+    float acc = 0.f;
+    if (i < kPartLoss) {
+        int b = b0;
+        for (; b + 8 <= b1; b += 8) {
+            float t[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) t[u] = __ldcs(part + (size_t)(b + u) * kPartSize + i);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) acc += t[u];
+        }
+        for (; b < b1; ++b) acc += __ldcs(part + (size_t)b * kPartSize + i);
+    }
+    sums[w][lane] = acc;
+    __syncthreads();
+    if (w != 0 || i >= kPartLoss) return;
     float gsum = 0.f;
-    for (int b = 0; b < nblocks; ++b) gsum += part[(size_t)b * kPartSize + i];
+#pragma unroll
+    for (int u = 0; u < kAdamWarps; ++u) gsum += sums[u][lane];
     // masked entries: the unused input column 15, unused outputs 3..7
     bool used = true;
-    float* w = nullptr;
+    float* wp = nullptr;
     bool decay = true;
     if (i < kPartW2) {
         const int in = i / kHid;
         used = in < 15;
-        w = p.W1 + i;
+        wp = p.W1 + i;
     } else if (i < kPartW3) {
-        w = p.W2 + (i - kPartW2);
+        wp = p.W2 + (i - kPartW2);
     } else if (i < kPartB1) {
         const int o = (i - kPartW3) % kOut;
         used = o < kOutUsed;
-        w = p.W3 + (i - kPartW3);
+        wp = p.W3 + (i - kPartW3);
     } else if (i < kPartB2) {
-        w = p.b1 + (i - kPartB1);
+        wp = p.b1 + (i - kPartB1);
         decay = false;
     } else if (i < kPartB3) {
-        w = p.b2 + (i - kPartB2);
+        wp = p.b2 + (i - kPartB2);
         decay = false;
     } else {
         const int o = i - kPartB3;
         used = o < kOutUsed;
-        w = p.b3 + o;
+        wp = p.b3 + o;
         decay = false;
     }
     if (grad_out) grad_out[i] = used ? gsum : 0.f;
@@ -424,10 +523,10 @@ __global__ void k_mlp_adamw(MlpParams p, const float* __restrict__ part, int nbl
     m[i] = beta1 * m[i] + (1.f - beta1) * gsum;
     v[i] = beta2 * v[i] + (1.f - beta2) * gsum * gsum;
     const float mh = m[i] / b1c, vh = v[i] / b2c;
-    float wv = *w;
+    float wv = *wp;
     if (decay) wv -= lr * wd * wv;
     wv -= lr * mh / (sqrtf(vh) + eps);
-    *w = wv;
+    *wp = wv;
 }
 
 __global__ void k_mlp_pack(MlpParams p) {
@@ -453,6 +552,7 @@ __global__ void k_mlp_pack(MlpParams p) {
 
 }  // namespace
 
+static_assert(sizeof(SmemTrain) <= 227 * 1024, "shared memory of the training kernel");
 size_t mlp_forward_smem() { return sizeof(Smem); }
 size_t mlp_train_smem() { return sizeof(SmemTrain); }
 
@@ -475,7 +575,7 @@ int launch_mlp_train(const MlpParams& p, const void* X, const float* Y, int n, f
 
 void launch_mlp_adamw(const MlpParams& p, const float* part, int nblocks, float lr, float b1, float b2, float eps,
                       float wd, int step, float* m, float* v, float* grad_out, float* loss_out, cudaStream_t st) {
-    k_mlp_adamw<<<(kPartLoss + 255) / 256, 256, 0, st>>>(p, part, nblocks, lr, b1, b2, eps, wd, step, m, v, grad_out,
+    k_mlp_adamw<<<(kPartLoss + 31) / 32 + 1, 32 * kAdamWarps, 0, st>>>(p, part, nblocks, lr, b1, b2, eps, wd, step, m, v, grad_out,
                                                          loss_out);
     k_mlp_pack<<<(kHid * kHid + 255) / 256, 256, 0, st>>>(p);
 }

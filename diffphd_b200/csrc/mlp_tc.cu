@@ -2,15 +2,18 @@
 // tensor cores: tcgen05.mma with
 // BF16 operands in shared memory, FP32 accumulators in tensor memory (TMEM), read back with tcgen05.ld.
 //
-// One CTA of 128 threads works on tiles of 128 rows (nodes); thread t owns row t, which is TMEM lane t of every
-// accumulator (M = 128, cta_group::1).  Per tile:
+// One CTA of 512 threads works on tiles of 128 rows (nodes).  Row r is TMEM lane r of every accumulator (M = 128,
+// cta_group::1); a warp reaches the 32 lanes of its position in its warpgroup, so the four warpgroups take the same rows
+// and a quarter (32) of the hidden columns each.  Per tile:
 //   layer 1: D1[128 x 128] = X[128 x 16] W1^T        1 MMA  (K = 16 per instruction)
 //   layer 2: D2[128 x 128] = gelu(D1 + b1) W2^T       8 MMAs
 //   layer 3: D3[128 x 16]  = gelu(D2 + b2) W3^T       8 MMAs (N = 16: outputs 0..7 used, 8..15 zero rows)
-// Between layers each thread reads its row of the accumulator (tcgen05.ld 32x32b), adds the bias, applies
-// GELU, rounds to BF16 and writes the row into the next layer's A tile; thread 0 issues the
-// MMAs and commits them to an mbarrier that every thread waits on (bounded).  The weights are staged into
-// shared memory once per CTA; CTAs loop over tiles.
+// Between layers each thread reads its 32 columns of its row of the accumulator (tcgen05.ld 32x32b), adds the bias,
+// applies GELU, rounds to BF16 and writes them into the next layer's A tile; thread 0 issues the MMAs and commits them to
+// an mbarrier that every thread waits on (bounded).  The weights are staged into shared memory once per CTA; CTAs loop
+// over tiles, and a tile's X rows are fetched during the tile before.  What bounds it is the issue of the GELU's
+// arithmetic (256 erff a row): with one thread a row, two CTAs an SM had 8 warps to hide its latencies and the MMA waits
+// (274,625 rows: 133 us, now 90; 425 rows: 18.7 us, now 12.5).
 //
 // Shared-memory operands use the K-major, no-swizzle canonical layout of the UMMA descriptors: "core matrices"
 // of 8 rows x 16 bytes (8 BF16 along K) stored contiguously (128 B), ordered [k / 8][row / 8].  For the MMA of
@@ -27,7 +30,8 @@ namespace dphd {
 
 namespace {
 
-constexpr int kTcRows = 128;                     // M: rows per tile, one per thread
+constexpr int kTcRows = 128;                     // M: rows per tile
+constexpr int kTcThreads = 512;
 constexpr int kIn = 16, kHid = 128, kOut8 = 8, kN3 = 16;
 constexpr uint32_t kTmemCols = 128;              // one FP32 accumulator of N <= 128 columns
 constexpr long long kWaitPolls = 1ll << 22;      // bound of every mbarrier wait
@@ -162,7 +166,7 @@ __device__ __forceinline__ void gelu_to_tile(const float* v, const float* bias, 
     }
 }
 
-__global__ void __launch_bounds__(128) k_mlp_forward_tc(const __nv_bfloat16* __restrict__ W1T,
+__global__ void __launch_bounds__(kTcThreads, 2) k_mlp_forward_tc(const __nv_bfloat16* __restrict__ W1T,
                                                         const __nv_bfloat16* __restrict__ W2T,
                                                         const __nv_bfloat16* __restrict__ W3T,
                                                         const float* __restrict__ b1, const float* __restrict__ b2,
@@ -206,7 +210,8 @@ __global__ void __launch_bounds__(128) k_mlp_forward_tc(const __nv_bfloat16* __r
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem = s.tmem_base;
-    const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);  // this warp's 32 TMEM lanes
+    const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);  // this warp's 32 TMEM lanes
+    const int lr = t & (kTcRows - 1), c0 = (t / kTcRows) * 32;              // its row and first hidden column
     const uint32_t id128 = make_idesc(kTcRows, kHid), id16 = make_idesc(kTcRows, kN3);
     const uint32_t a1 = smem_addr(s.A1), a2 = smem_addr(s.A2), bb1 = smem_addr(s.B1), bb2 = smem_addr(s.B2),
                    bb3 = smem_addr(s.B3);
@@ -231,16 +236,16 @@ __global__ void __launch_bounds__(128) k_mlp_forward_tc(const __nv_bfloat16* __r
         fence_after_sync();
     };
     const int ntiles = (n + kTcRows - 1) / kTcRows;
+    // X tile: the first 256 threads fetch one 16-byte core row (8 of a row's 16 BF16) each, zero beyond n
+    const int xr = t >> 1, xk = (t & 1) * 8;
+    auto fetch_x = [&](int tile) {
+        const long long row = (long long)tile * kTcRows + xr;
+        return t < 2 * kTcRows && row < n ? *reinterpret_cast<const uint4*>(X + row * kIn + xk) : make_uint4(0, 0, 0, 0);
+    };
+    uint4 x = fetch_x(blockIdx.x);
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int row = tile * kTcRows + t;
-        // X tile: this thread's row (16 BF16 = two 16-byte core rows), zero beyond n
-        uint4 x0 = make_uint4(0, 0, 0, 0), x1 = make_uint4(0, 0, 0, 0);
-        if (row < n) {
-            x0 = *reinterpret_cast<const uint4*>(X + (size_t)row * kIn);
-            x1 = *reinterpret_cast<const uint4*>(X + (size_t)row * kIn + 8);
-        }
-        *reinterpret_cast<uint4*>(s.A1 + cm_off(t, 0, kTcRows)) = x0;
-        *reinterpret_cast<uint4*>(s.A1 + cm_off(t, 8, kTcRows)) = x1;
+        const int row = tile * kTcRows + lr;
+        if (t < 2 * kTcRows) *reinterpret_cast<uint4*>(s.A1 + cm_off(xr, xk, kTcRows)) = x;
         publish();
         // layer 1: one K = 16 slice
         if (t == 0) {
@@ -248,12 +253,10 @@ __global__ void __launch_bounds__(128) k_mlp_forward_tc(const __nv_bfloat16* __r
             mma_commit(mbar);
         }
         if (!(ok = wait_mma())) break;
+        x = fetch_x(tile + gridDim.x);
         float v[32];
-#pragma unroll
-        for (int c0 = 0; c0 < kHid; c0 += 32) {
-            tmem_ld32(lane_addr + c0, v);
-            gelu_to_tile(v, s.b1, c0, t, s.A2);
-        }
+        tmem_ld32(lane_addr + c0, v);
+        gelu_to_tile(v, s.b1, c0, lr, s.A2);
         publish();
         // layer 2: eight K-slices of 16
         if (t == 0) {
@@ -265,11 +268,8 @@ __global__ void __launch_bounds__(128) k_mlp_forward_tc(const __nv_bfloat16* __r
         }
         if (!(ok = wait_mma())) break;
         // layer 2 has finished reading A2: the layer-3 input overwrites it
-#pragma unroll
-        for (int c0 = 0; c0 < kHid; c0 += 32) {
-            tmem_ld32(lane_addr + c0, v);
-            gelu_to_tile(v, s.b2, c0, t, s.A2);
-        }
+        tmem_ld32(lane_addr + c0, v);
+        gelu_to_tile(v, s.b2, c0, lr, s.A2);
         publish();
         // layer 3: N = 16 (rows 8..15 of W3^T are zero)
         if (t == 0) {
@@ -280,6 +280,7 @@ __global__ void __launch_bounds__(128) k_mlp_forward_tc(const __nv_bfloat16* __r
             mma_commit(mbar);
         }
         if (!(ok = wait_mma())) break;
+        if (warp >= 4) continue;  // the first warpgroup reads the 16 output columns
         tmem_ld16(lane_addr, v);
         if (row < n) {
             float4* o = reinterpret_cast<float4*>(out + (size_t)row * kOut8);
@@ -320,7 +321,7 @@ void launch_mlp_forward_tc(const void* W1T, const void* W2T, const void* W3T, co
     const int smem = (int)mlp_tc_smem();
     cudaFuncSetAttribute(k_mlp_forward_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     const int grid = ntiles < max_ctas ? ntiles : max_ctas;
-    k_mlp_forward_tc<<<grid, 128, smem, st>>>(
+    k_mlp_forward_tc<<<grid, kTcThreads, smem, st>>>(
         reinterpret_cast<const __nv_bfloat16*>(W1T), reinterpret_cast<const __nv_bfloat16*>(W2T),
         reinterpret_cast<const __nv_bfloat16*>(W3T), b1, b2, b3, reinterpret_cast<const __nv_bfloat16*>(X), n, out,
         err, g_mma_wait_polls);
