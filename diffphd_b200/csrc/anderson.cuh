@@ -1,4 +1,4 @@
-// The Type-II Anderson system (forward_gpu.cpp:1340-1379), solved by one thread.
+// The Type-II Anderson system (forward_gpu.cpp:1340-1379), solved by one warp.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -6,97 +6,84 @@
 
 namespace dphd {
 
-constexpr int kAaVals = 2 * kMaxWindow + 2;  // new Gram column, right-hand side, |g|^2, |x_raw|^2
+constexpr int kAaVals = 2 * kMaxWindow + 2;  // sums of an iteration, at most
+// Shared memory of the solve.  tot: the new difference's Gram column (m entries), dG^T g (m), |g|^2, |x_raw|^2.
+struct AaSystem {
+    double tot[kAaVals];
+    double A[kMaxWindow][kMaxWindow + 1], b[kMaxWindow], inv[kMaxWindow], gamma[kMaxWindow];
+    int accept, restart;
+};
 
-// tot: the new difference's Gram column (j < m) and, from kMaxWindow on, dG^T g; gram by ring slot.  Sets `accept` with
-// gamma, or `restart`.
-__device__ __forceinline__ void aa_solve(const double* tot, int m, int head, int W, double (*gram)[kMaxWindow],
-                                         double* gamma, int* accept, int* restart) {
-    // Extend the stored Gram matrix by the new difference's column, then solve
-    // (dG^T dG + reg I) gamma = dG^T g, reg = max(1e-6 |dG|_F^2 / m, 1e-12), by Cholesky.  All loops run to
-    // kMaxWindow with guards so that the small arrays stay in registers; the stored entries are loaded
-    // independently (one round trip) rather than inside the factorisation.
-    const int snew = (head + m - 1) % W;
-    double A[kMaxWindow][kMaxWindow], b[kMaxWindow];
-#pragma unroll
-    for (int i = 0; i < kMaxWindow; ++i)
-#pragma unroll
-        for (int j = 0; j < kMaxWindow; ++j)
-            if (i < m && j < m)
-                A[i][j] = (i == m - 1) ? tot[j] : (j == m - 1) ? tot[i] : gram[(head + i) % W][(head + j) % W];
-#pragma unroll
-    for (int j = 0; j < kMaxWindow; ++j)
-        if (j < m) {
-            const int sj = (head + j) % W;
-            gram[snew][sj] = tot[j];
-            gram[sj][snew] = tot[j];
-        }
-    double fro = 0;
-#pragma unroll
-    for (int j = 0; j < kMaxWindow; ++j)
-        if (j < m) fro += A[j][j];
-    const double reg = fmax(1e-6 * fro / m, 1e-12);
-#pragma unroll
-    for (int i = 0; i < kMaxWindow; ++i)
-        if (i < m) {
-            A[i][i] += reg;
-            b[i] = tot[kMaxWindow + i];
-        }
-    // one reciprocal per column (a single thread runs this: FP64 divisions dominate its latency)
-    double inv_diag[kMaxWindow];
-#pragma unroll
-    for (int j = 0; j < kMaxWindow; ++j) {
-        inv_diag[j] = 0.0;
-        if (j < m) {
-            double d = A[j][j];
-#pragma unroll
-            for (int k = 0; k < kMaxWindow; ++k)
-                if (k < j) d -= A[j][k] * A[j][k];
-            d = sqrt(fmax(d, 1e-300));
-            A[j][j] = d;
-            const double inv = 1.0 / d;
-            inv_diag[j] = inv;
-#pragma unroll
-            for (int i = 0; i < kMaxWindow; ++i)
-                if (i > j && i < m) {
-                    double t = A[i][j];
-#pragma unroll
-                    for (int k = 0; k < kMaxWindow; ++k)
-                        if (k < j) t -= A[i][k] * A[j][k];
-                    A[i][j] = t * inv;
-                }
-        }
+// Extends the Gram matrix (by ring slot) by the new difference's column, then solves (dG^T dG + reg I) gamma = dG^T g,
+// reg = max(1e-6 |dG|_F^2 / m, 1e-12), by Cholesky, lane i on row i: sets `accept` with gamma, or `restart`.  The loops
+// stay rolled: this runs once per iteration, so its code comes from the outer instruction caches, and unrolled to the
+// largest window it took a single thread 128 registers and 9 us.
+__device__ __forceinline__ void aa_solve_warp(AaSystem& s, double (*gram)[kMaxWindow], int m, int head, int W, int lane) {
+    const int snew = (head + m - 1) % W, si = (head + lane) % W;
+    if (lane < m) {
+#pragma unroll 1
+        for (int j = 0; j < m; ++j)
+            s.A[lane][j] = (lane == m - 1) ? s.tot[j] : (j == m - 1) ? s.tot[lane] : gram[si][(head + j) % W];
+        s.b[lane] = s.tot[m + lane];
     }
-#pragma unroll
-    for (int i = 0; i < kMaxWindow; ++i)
-        if (i < m) {
-            double t = b[i];
-#pragma unroll
-            for (int k = 0; k < kMaxWindow; ++k)
-                if (k < i) t -= A[i][k] * b[k];
-            b[i] = t * inv_diag[i];
+    __syncwarp();
+    if (lane < m) {
+        gram[snew][si] = s.tot[lane];
+        gram[si][snew] = s.tot[lane];
+    }
+    double fro = 0;
+#pragma unroll 1
+    for (int j = 0; j < m; ++j) fro += s.A[j][j];
+    const double reg = fmax(1e-6 * fro / m, 1e-12);
+    __syncwarp();
+    if (lane < m) s.A[lane][lane] += reg;
+    __syncwarp();
+#pragma unroll 1
+    for (int j = 0; j < m; ++j) {
+        double t = 0.0;
+        if (lane >= j && lane < m) {
+            t = s.A[lane][j];
+#pragma unroll 1
+            for (int k = 0; k < j; ++k) t -= s.A[lane][k] * s.A[j][k];
         }
-#pragma unroll
-    for (int i = kMaxWindow - 1; i >= 0; --i)
-        if (i < m) {
-            double t = b[i];
-#pragma unroll
-            for (int k = 0; k < kMaxWindow; ++k)
-                if (k > i && k < m) t -= A[k][i] * b[k];
-            b[i] = t * inv_diag[i];
+        const double d = sqrt(fmax(__shfl_sync(0xffffffffu, t, j), 1e-300));
+        const double inv = 1.0 / d;
+        if (lane == j) {
+            s.A[j][j] = d;
+            s.inv[j] = inv;
+        } else if (lane > j && lane < m) {
+            s.A[lane][j] = t * inv;
         }
-    double gn = 0;
-#pragma unroll
-    for (int i = 0; i < kMaxWindow; ++i)
-        if (i < m) gn += b[i] * b[i];
-    gn = sqrt(gn);
-    if (!(gn < 10.0)) {
-        *restart = 1;
-    } else {
-        *accept = 1;
-#pragma unroll
-        for (int i = 0; i < kMaxWindow; ++i)
-            if (i < m) gamma[i] = b[i];
+        __syncwarp();
+    }
+    double t = lane < m ? s.b[lane] : 0.0;
+#pragma unroll 1
+    for (int k = 0; k < m; ++k) {  // L y = b
+        if (lane == k) t *= s.inv[k];
+        const double yk = __shfl_sync(0xffffffffu, t, k);
+        if (lane > k && lane < m) t -= s.A[lane][k] * yk;
+    }
+    if (lane < m) s.b[lane] = t;
+    __syncwarp();
+    if (lane == 0) {
+#pragma unroll 1
+        for (int i = m - 1; i >= 0; --i) {  // L^T x = y
+            double x = s.b[i];
+#pragma unroll 1
+            for (int k = i + 1; k < m; ++k) x -= s.A[k][i] * s.b[k];
+            s.b[i] = x * s.inv[i];
+        }
+        double gn = 0;
+#pragma unroll 1
+        for (int i = 0; i < m; ++i) gn += s.b[i] * s.b[i];
+        gn = sqrt(gn);
+        if (!(gn < 10.0)) {
+            s.restart = 1;
+        } else {
+            s.accept = 1;
+#pragma unroll 1
+            for (int i = 0; i < m; ++i) s.gamma[i] = s.b[i];
+        }
     }
 }
 

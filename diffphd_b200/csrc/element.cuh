@@ -45,20 +45,57 @@ __device__ __forceinline__ void def_grad(const int* __restrict__ E, int e, Ld x,
     }
 }
 
-// The 8 corners' contributions of the 8 consecutive lanes of a hex, summed over the lanes; lane l is left with corner l
-// in acc[0].  Each step hands the half of the corners that the partner keeps to it and adds the partner's: the same
-// pairs, in the same order, as a butterfly over all corners, with 21 exchanges instead of 72.
-__device__ __forceinline__ void sum_samples(double (*acc)[3], int smp) {
+// Contribution P g_a of a sample's corner a.
+__device__ __forceinline__ void corner(const double* P, const double* __restrict__ g, int a, double* c) {
+    const double g0 = __ldg(g + a * 3), g1 = __ldg(g + a * 3 + 1), g2 = __ldg(g + a * 3 + 2);
 #pragma unroll
-    for (int o = 4; o > 0; o >>= 1) {
+    for (int i = 0; i < 3; ++i) c[i] = P[i] * g0 + P[i + 3] * g1 + P[i + 6] * g2;
+}
+
+// The 8 corners' contributions of the 8 consecutive lanes (samples) of a hex, summed over the lanes; lane l is left with
+// corner l in acc.  Each step hands the half of the corners that the partner keeps to it and adds the partner's: the same
+// pairs, in the same order, as a butterfly over all corners, with 21 exchanges instead of 72, and the corners are formed
+// as the first step hands them over (12 live values instead of 24).
+__device__ __forceinline__ void sum_samples(const double* P, const double* __restrict__ g, int smp, double* acc) {
+    double c[4][3];
+    const int up4 = smp & 4;
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        double give[3];
+        corner(P, g, a + up4, c[a]);
+        corner(P, g, a + (up4 ^ 4), give);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) c[a][i] += __shfl_xor_sync(0xffffffffu, give[i], 4);
+    }
+#pragma unroll
+    for (int o = 2; o > 0; o >>= 1) {
         const bool up = (smp & o) != 0;
 #pragma unroll
         for (int a = 0; a < o; ++a)
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
-                const double keep = up ? acc[a + o][i] : acc[a][i], give = up ? acc[a][i] : acc[a + o][i];
-                acc[a][i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                const double keep = up ? c[a + o][i] : c[a][i], give = up ? c[a][i] : c[a + o][i];
+                c[a][i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
             }
+    }
+    acc[0] = c[0][0]; acc[1] = c[0][1]; acc[2] = c[0][2];
+}
+
+// Writes the sample's corner contributions P g_a to the element's slots (hexes: summed over the samples first; every lane
+// of the warp calls this).
+template <int K, int S>
+__device__ __forceinline__ void scatter_corners(const double* P, const double* __restrict__ g, int e, int smp, bool valid,
+                                                double* __restrict__ out) {
+    if constexpr (S == 8) {
+        double c[3];
+        sum_samples(P, g, smp, c);
+        if (valid) {
+            double* o = out + ((size_t)e * K + smp) * 3;
+            o[0] = c[0]; o[1] = c[1]; o[2] = c[2];
+        }
+    } else if (valid) {
+#pragma unroll
+        for (int a = 0; a < K; ++a) corner(P, g, a, out + ((size_t)e * K + a) * 3);
     }
 }
 
@@ -72,11 +109,11 @@ __device__ __forceinline__ void elem_fwd_sample(int t, int m, const int* __restr
                                                 const EnergyPack& ep, double* __restrict__ out, int* status) {
     const int e = t / S, smp = t % S;
     const bool valid = e < m;
-    double acc[K][3];
+    const double* g = (S == 8) ? grad + smp * 24 : grad + (size_t)e * 12;
+    double P[9];
 #pragma unroll
-    for (int a = 0; a < K; ++a) acc[a][0] = acc[a][1] = acc[a][2] = 0.0;
+    for (int i = 0; i < 9; ++i) P[i] = 0.0;
     if (valid) {
-        const double* g = (S == 8) ? grad + smp * 24 : grad + (size_t)e * 12;
         double Fd[9], Fbd[9];
         def_grad<K>(E, e, x, g, Fd);
         if (elem_dir[e]) def_grad<K>(E, e, LdPlain{qb}, g, Fbd);
@@ -89,9 +126,6 @@ __device__ __forceinline__ void elem_fwd_sample(int t, int m, const int* __restr
         for (int i = 0; i < 9; ++i) F[i] = (T)Fd[i];
         T U[9], V[9], sig[3];
         svd3<T>(F, U, sig, V);
-        double P[9];
-#pragma unroll
-        for (int i = 0; i < 9; ++i) P[i] = 0.0;
         bool ok = true;
         for (int k = 0; k < ep.count; ++k) {
             const ElemEnergyDev& en = ep.en[k];
@@ -109,26 +143,8 @@ __device__ __forceinline__ void elem_fwd_sample(int t, int m, const int* __restr
             }
         }
         if (!ok) atomicOr(status, (int)kStatusSingularF);
-#pragma unroll
-        for (int a = 0; a < K; ++a) {
-            const double g0 = __ldg(g + a * 3), g1 = __ldg(g + a * 3 + 1), g2 = __ldg(g + a * 3 + 2);
-#pragma unroll
-            for (int i = 0; i < 3; ++i) acc[a][i] = P[i] * g0 + P[i + 3] * g1 + P[i + 6] * g2;
-        }
     }
-    if constexpr (S == 8) {
-        sum_samples(acc, smp);
-        if (valid) {
-            double* o = out + ((size_t)e * K + smp) * 3;
-            o[0] = acc[0][0]; o[1] = acc[0][1]; o[2] = acc[0][2];
-        }
-    } else if (valid) {
-#pragma unroll
-        for (int a = 0; a < K; ++a) {
-            double* o = out + ((size_t)e * K + a) * 3;
-            o[0] = acc[a][0]; o[1] = acc[a][1]; o[2] = acc[a][2];
-        }
-    }
+    scatter_corners<K, S>(P, g, e, smp, valid, out);
 }
 
 // The cached Jacobians are stored by blocks of 32 samples, entry by entry within a block (entry k of sample t at
@@ -145,44 +161,23 @@ __device__ __forceinline__ void kpd_sample(int t, int m, const int* __restrict__
                                            double* __restrict__ out) {
     const int e = t / S, smp = t % S;
     const bool valid = e < m;
-    double acc[K][3];
+    const double* g = (S == 8) ? grad + smp * 24 : grad + (size_t)e * 12;
+    double P[9];
 #pragma unroll
-    for (int a = 0; a < K; ++a) acc[a][0] = acc[a][1] = acc[a][2] = 0.0;
+    for (int i = 0; i < 9; ++i) P[i] = 0.0;
     if (valid) {
-        const double* g = (S == 8) ? grad + smp * 24 : grad + (size_t)e * 12;
         double dF[9];
         def_grad<K>(E, e, x, g, dF);
         constexpr int N = kJStride;
         const double* Jt = J + j_base(t, 81);
-        double P[9];
-#pragma unroll
-        for (int i = 0; i < 9; ++i) P[i] = 0.0;
 #pragma unroll
         for (int col = 0; col < 9; ++col) {
             const double f = dF[col];
 #pragma unroll
             for (int i = 0; i < 9; ++i) P[i] += __ldg(Jt + (col * 9 + i) * N) * f;
         }
-#pragma unroll
-        for (int a = 0; a < K; ++a) {
-            const double g0 = __ldg(g + a * 3), g1 = __ldg(g + a * 3 + 1), g2 = __ldg(g + a * 3 + 2);
-#pragma unroll
-            for (int i = 0; i < 3; ++i) acc[a][i] = P[i] * g0 + P[i + 3] * g1 + P[i + 6] * g2;
-        }
     }
-    if constexpr (S == 8) {
-        sum_samples(acc, smp);
-        if (valid) {
-            double* o = out + ((size_t)e * K + smp) * 3;
-            o[0] = acc[0][0]; o[1] = acc[0][1]; o[2] = acc[0][2];
-        }
-    } else if (valid) {
-#pragma unroll
-        for (int a = 0; a < K; ++a) {
-            double* o = out + ((size_t)e * K + a) * 3;
-            o[0] = acc[a][0]; o[1] = acc[a][1]; o[2] = acc[a][2];
-        }
-    }
+    scatter_corners<K, S>(P, g, e, smp, valid, out);
 }
 
 }  // namespace dphd

@@ -32,11 +32,9 @@ struct Smem {
     int slot[2][kSmallChunk];
     double y[2][3][kSmallChunk];
     double sh[kAaVals][32];   // per-warp sums: Gram column (m), right-hand side (m), |g|^2, |x_raw|^2
-    double tot[kAaVals];      // their totals
     double tot2[5];
     double gram[kMaxWindow][kMaxWindow];
-    double A[kMaxWindow][kMaxWindow + 1], b[kMaxWindow], inv[kMaxWindow], gamma[kMaxWindow];
-    int accept, restart;
+    AaSystem aa;
 };
 
 __device__ __forceinline__ void cluster_sync() {
@@ -127,78 +125,6 @@ __device__ __forceinline__ void s_rows(const SpmvPlan<double>& p, const double* 
     const double tot = t[0] + __shfl_xor_sync(0xffffffffu, t[0], 1);
     if ((lane & 1) == 0 && idx < 3 * nr)
         p.ypart[(size_t)__ldg(p.unit_item_slot + first + idx / 3) * 3 + idx % 3] = tot;
-}
-
-// aa_solve by one warp, lane i on row i: every entry is formed by the same subtractions in the same order as there.  The
-// loops stay rolled: every phase of this kernel runs once per iteration, so its code comes from the instruction caches'
-// outer levels, and fewer instructions are fetched this way.
-__device__ __forceinline__ void aa_solve_warp(Smem& s, int m, int head, int W, int lane) {
-    const int snew = (head + m - 1) % W, si = (head + lane) % W;
-    if (lane < m) {
-#pragma unroll 1
-        for (int j = 0; j < m; ++j)
-            s.A[lane][j] = (lane == m - 1) ? s.tot[j] : (j == m - 1) ? s.tot[lane] : s.gram[si][(head + j) % W];
-        s.b[lane] = s.tot[m + lane];
-    }
-    __syncwarp();
-    if (lane < m) {
-        s.gram[snew][si] = s.tot[lane];
-        s.gram[si][snew] = s.tot[lane];
-    }
-    double fro = 0;
-#pragma unroll 1
-    for (int j = 0; j < m; ++j) fro += s.A[j][j];
-    const double reg = fmax(1e-6 * fro / m, 1e-12);
-    __syncwarp();
-    if (lane < m) s.A[lane][lane] += reg;
-    __syncwarp();
-#pragma unroll 1
-    for (int j = 0; j < m; ++j) {
-        double t = 0.0;
-        if (lane >= j && lane < m) {
-            t = s.A[lane][j];
-#pragma unroll 1
-            for (int k = 0; k < j; ++k) t -= s.A[lane][k] * s.A[j][k];
-        }
-        const double d = sqrt(fmax(__shfl_sync(0xffffffffu, t, j), 1e-300));
-        const double inv = 1.0 / d;
-        if (lane == j) {
-            s.A[j][j] = d;
-            s.inv[j] = inv;
-        } else if (lane > j && lane < m) {
-            s.A[lane][j] = t * inv;
-        }
-        __syncwarp();
-    }
-    double t = lane < m ? s.b[lane] : 0.0;
-#pragma unroll 1
-    for (int k = 0; k < m; ++k) {  // L y = b
-        if (lane == k) t *= s.inv[k];
-        const double yk = __shfl_sync(0xffffffffu, t, k);
-        if (lane > k && lane < m) t -= s.A[lane][k] * yk;
-    }
-    if (lane < m) s.b[lane] = t;
-    __syncwarp();
-    if (lane == 0) {
-#pragma unroll 1
-        for (int i = m - 1; i >= 0; --i) {  // L^T x = y
-            double x = s.b[i];
-#pragma unroll 1
-            for (int k = i + 1; k < m; ++k) x -= s.A[k][i] * s.b[k];
-            s.b[i] = x * s.inv[i];
-        }
-        double gn = 0;
-#pragma unroll 1
-        for (int i = 0; i < m; ++i) gn += s.b[i] * s.b[i];
-        gn = sqrt(gn);
-        if (!(gn < 10.0)) {
-            s.restart = 1;
-        } else {
-            s.accept = 1;
-#pragma unroll 1
-            for (int i = 0; i < m; ++i) s.gamma[i] = s.b[i];
-        }
-    }
 }
 
 template <int K, int S, int MODE>
@@ -438,24 +364,24 @@ __global__ void __launch_bounds__(kThr, 1) k_small_loop(SmallLoop a, int cap) {
 #pragma unroll 1
         for (int i = wid; i < nv; i += kThr / 32) {
             const double t = total_of(a.part_aa + i, nblk, kAaVals, lane);
-            if (lane == 0) s.tot[i] = t;
+            if (lane == 0) s.aa.tot[i] = t;
         }
         __syncthreads();
-        err = sqrt(s.tot[2 * m]);
-        xraw_norm = sqrt(s.tot[2 * m + 1]);
+        err = sqrt(s.aa.tot[2 * m]);
+        xraw_norm = sqrt(s.aa.tot[2 * m + 1]);
         const bool diverged = MODE == 1 && (!(xraw_norm == xraw_norm) || xraw_norm > 1e300 ||
                                             (clip > 0 && xraw_norm > clip));
         if (diverged)
             status |= (xraw_norm == xraw_norm && xraw_norm <= 1e300) ? (int)kStatusDiverged
                                                                      : (int)(kStatusDiverged | kStatusNonFinite);
         if (wid == 0) {
-            if (lane == 0) s.accept = s.restart = 0;
+            if (lane == 0) s.aa.accept = s.aa.restart = 0;
             __syncwarp();
-            if (!diverged && m >= 1) aa_solve_warp(s, m, head, W, lane);
+            if (!diverged && m >= 1) aa_solve_warp(s.aa, s.gram, m, head, W, lane);
         }
         __syncthreads();
         // ---- extrapolation, Dirichlet values, gate (k_aa_update's blocks) ----
-        const int accept = s.accept, restart = s.restart;
+        const int accept = s.aa.accept, restart = s.aa.restart;
         double u3[3] = {0.0, 0.0, 0.0};
         if (own) {
             double xn = xv;
@@ -463,7 +389,7 @@ __global__ void __launch_bounds__(kThr, 1) k_small_loop(SmallLoop a, int cap) {
 #pragma unroll 1
                 for (int j = 0; j < m; ++j) {
                     const int sl = (head + j) % W;
-                    xn -= (s.hist[kMaxWindow + sl][ht] + s.hist[sl][ht]) * s.gamma[j];
+                    xn -= (s.hist[kMaxWindow + sl][ht] + s.hist[sl][ht]) * s.aa.gamma[j];
                 }
                 if (fx) xn = fv;
             }
