@@ -22,6 +22,7 @@
 
 #include "dphd_internal.h"
 #include "kernels.cuh"
+#include "launch.cuh"
 
 namespace dphd {
 
@@ -58,6 +59,7 @@ void* scratch_address() {
 template <typename T>
 __global__ void k_noalloc_prepare(int n, int npad, const double* __restrict__ b, const unsigned char* __restrict__ fixed,
                                   const int* __restrict__ perm, size_t ctrl_off, size_t v_off) {
+    pdl_enter();  // a call may follow another one's kernels, which read the array this one writes
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < (int)(sizeof(Ctrl) / sizeof(int))) reinterpret_cast<int*>(g_noalloc_scratch + ctrl_off)[t] = 0;
     if (t >= npad) return;
@@ -101,7 +103,7 @@ void run(const SpmvPlan<T>& plan, const unsigned char* fixed_node, const double*
     p.row_cnt = nullptr;
     const Ctrl* ctrl = reinterpret_cast<const Ctrl*>(base + ctrl_off);
     const int threads = 256, blocks = (std::max(npad, 64) + threads - 1) / threads;
-    k_noalloc_prepare<T><<<blocks, threads, 0, st>>>(n, npad, d_b, fixed_node, plan.perm, ctrl_off, v_off);
+    launch_k(k_noalloc_prepare<T>, blocks, threads, 0, st, n, npad, d_b, fixed_node, plan.perm, ctrl_off, v_off);
     launch_sts<T>(p, reinterpret_cast<const T*>(base + v_off), reinterpret_cast<T*>(base + y_off), d_x, ctrl, st);
     const cudaError_t e = cudaGetLastError();
     DPHD_CHECK(e == cudaSuccess, std::string("dphd_ainv_noalloc launch failed: ") + cudaGetErrorString(e));

@@ -173,10 +173,20 @@ __global__ void __launch_bounds__(kThr, 1) k_small_loop(SmallLoop a, int cap) {
         double g0 = 0.0, g1 = 0.0;
         for (int base = gw * (32 / kGatherLanes); base < n; base += kThreads / kGatherLanes) {
             const int i = base + lane / kGatherLanes, gl = lane & (kGatherLanes - 1);
-            const bool valid = i < n;
-            double p[3] = {0.0, 0.0, 0.0};
+            const bool valid = i < n, out = valid && gl < 3;  // lane d of a node's group finishes component d
+            const int o = 3 * i + gl;
+            double p[3] = {0.0, 0.0, 0.0}, pr = 0.0, rhs = 0.0;
+            int j = 0;
+            bool fix = false;
+            if (out) {  // in flight together with the sums' loads
+                j = a.iperm[i];
+                fix = a.fixed_node[i] != 0;
+                rhs = a.rhs[o];
+                if (MODE == 0) pr = a.prev[o];
+            }
             if (valid) {
                 const int e = a.node_ptr[i + 1];
+#pragma unroll 1
                 for (int idx = a.node_ptr[i] + gl; idx < e; idx += 4 * kGatherLanes) {
                     int k[4];
                     double c[4][3];
@@ -197,23 +207,18 @@ __global__ void __launch_bounds__(kThr, 1) k_small_loop(SmallLoop a, int cap) {
             }
 #pragma unroll
             for (int d = 0; d < 3; ++d) p[d] = gsum8(p[d]);
-            if (valid && gl == 0) {
-                const int j = a.iperm[i];
-                const bool fix = a.fixed_node[i] != 0;
-#pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    double val;
-                    if (MODE == 0) {
-                        const double pr = a.prev[3 * i + d];
-                        g0 += (p[d] - pr) * (p[d] - pr);
-                        g1 += pr * pr;
-                        a.prev[3 * i + d] = p[d];
-                        val = fix ? 0.0 : a.inv_h2m * a.rhs[3 * i + d] + p[d];
-                    } else {
-                        val = fix ? 0.0 : a.rhs[3 * i + d] + p[d];
-                    }
-                    a.v[(size_t)d * npad + j] = val;
+            if (out) {
+                const double pd = gl == 0 ? p[0] : gl == 1 ? p[1] : p[2];
+                double val;
+                if (MODE == 0) {
+                    g0 += (pd - pr) * (pd - pr);
+                    g1 += pr * pr;
+                    a.prev[o] = pd;
+                    val = fix ? 0.0 : a.inv_h2m * rhs + pd;
+                } else {
+                    val = fix ? 0.0 : rhs + pd;
                 }
+                a.v[(size_t)gl * npad + j] = val;
             }
         }
         if (MODE == 0) {  // |d pd|^2, |pd|^2 of this CTA
