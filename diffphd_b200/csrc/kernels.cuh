@@ -196,8 +196,8 @@ struct SmallLoop {
     Ctrl* ctrl = nullptr;
 };
 // The rule of this path: us per iteration, launched loop -> one kernel, forward | adjoint:
-//   63 nodes 43 -> 31 | 41 -> 25     425 nodes 49 -> 40 | 44 -> 23     714 nodes (3,840 samples) 51 -> 47 | 41 -> 28
-//   800 nodes (2,835 tets) 55 -> 53 | 43 -> 29     1,053 nodes 57 -> 61 | 44 -> 37: 16 SMs no longer suffice
+//   63 nodes 43 -> 27 | 41 -> 19     425 nodes 49 -> 30 | 44 -> 18     714 nodes (3,840 samples) 51 -> 37 | 41 -> 24
+//   800 nodes (2,835 tets) 55 -> 44 | 43 -> 27     1,053 nodes 57 -> 57 | 44 -> 38: 16 SMs no longer suffice
 constexpr int kSmallChunk = 64;       // largest S^T chunk
 constexpr int kSmallDofs = 10 * 256;  // one degree of freedom per thread of the Anderson blocks, at most 16 of them
 constexpr int kSmallSamples = 4096;

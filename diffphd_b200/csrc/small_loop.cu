@@ -2,10 +2,10 @@
 //
 // A mesh of a few hundred nodes gives the iteration's eight launches almost nothing to do: on 425 nodes an iteration
 // took 49 us (forward) and 42 us (adjoint), nearly all of it launch and drain of grids of 5 to 64 CTAs.  Here one
-// cluster of 16 CTAs x 512 threads runs every iteration of the solve; the phases are separated by cluster barriers
+// cluster of 16 CTAs x 256 threads runs every iteration of the solve; the phases are separated by cluster barriers
 // (hardware, a few hundred ns), the Anderson history stays in shared memory and registers, and every CTA takes the
-// stop decision itself from the same sums.  What bounds it now is latency: the SVD's dependent divisions and roots (11
-// of 40 us forward), each phase's chain of L2 loads, and fetching each phase's code anew in every iteration.
+// stop decision itself from the same sums.  What bounds it now is latency: the SVD's dependent divisions and roots (10
+// of 30 us forward), each phase's chain of L2 loads, and fetching each phase's code anew in every iteration.
 //
 // Phases: element terms | node gather to the permuted right-hand side | y = S v by row groups | S^T column chunks |
 // x_raw, Anderson sums | extrapolation, gate.  Every value is formed by the expressions and in the order of the kernels
@@ -22,15 +22,15 @@ namespace dphd {
 
 namespace {
 
-constexpr int kCtas = 16, kThr = 512, kBlk = 256;  // kBlk: the launched loop's block of the Anderson sums and chunks
+constexpr int kCtas = 16, kThr = 256;  // the launched loop's block of the Anderson sums and of the S^T chunks
 
 struct Smem {
-    double hist[2 * kMaxWindow][kBlk];  // differences dG, dX by ring slot, of this CTA's block of degrees of freedom
-    double red[2][8][3][kTileCols];     // S^T chunk sums of the two half-CTAs
-    int2 cl[2][kSmallChunk];
-    long long off[2][kSmallChunk];
-    int slot[2][kSmallChunk];
-    double y[2][3][kSmallChunk];
+    double hist[2 * kMaxWindow][kThr];  // differences dG, dX by ring slot, of this CTA's block of degrees of freedom
+    double red[8][3][kTileCols];        // S^T chunk sums by warp
+    int2 cl[kSmallChunk];
+    long long off[kSmallChunk];
+    int slot[kSmallChunk];
+    double y[3][kSmallChunk];
     double sh[kAaVals][32];   // per-warp sums: Gram column (m), right-hand side (m), |g|^2, |x_raw|^2
     double tot2[5];
     double gram[kMaxWindow][kMaxWindow];
@@ -132,19 +132,18 @@ __global__ void __launch_bounds__(kThr, 1) k_small_loop(SmallLoop a, int cap) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Smem& s = *reinterpret_cast<Smem*>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int cta = blockIdx.x, half = tid / kBlk, ht = tid % kBlk, hw = ht >> 5;
+    const int cta = blockIdx.x;
     const int gw = wid * kCtas + cta;  // warps are dealt to the CTAs in turn, so that few warps' work uses every SM
     constexpr int kThreads = kCtas * kThr, kWarps = kThreads / 32;
     const int n = a.n, n3 = 3 * n, npad = a.p.npad;
     const int samples = a.m * S, sample_span = (samples + 31) / 32 * 32;
-    const int nblk = (n3 + kBlk - 1) / kBlk;  // <= kCtas
+    const int nblk = (n3 + kThr - 1) / kThr;  // <= kCtas
     Ctrl* const ctrl = a.ctrl;
     const int W = ctrl->window, max_iter = ctrl->max_iter;
     const double rel_tol = ctrl->rel_tol, abs_tol = ctrl->abs_tol, clip = ctrl->clip;
     int count = 0, head = 0, iter = 0, converged = 0, status = 0, loops = 0;
-    // this thread's degree of freedom (first half-CTA)
-    const int r = cta * kBlk + ht;
-    const bool own = half == 0 && cta < nblk && r < n3;
+    const int r = cta * kThr + tid;  // this thread's degree of freedom
+    const bool own = r < n3;
     double xp = 0.0, lg = 0.0, lx = 0.0, fv = 0.0;
     bool fx = false;
     int c0 = 0, c1 = 0, col = 0;
@@ -238,26 +237,20 @@ __global__ void __launch_bounds__(kThr, 1) k_small_loop(SmallLoop a, int cap) {
         // ---- y = S v ----
         for (int w = gw; w < a.p.n_units * (kUnitRows / kWarpRows); w += kWarps) s_rows(a.p, a.v, w, lane);
         cluster_sync();
-        // ---- S^T chunks: one per half-CTA (k_spmv_ST_part's order) ----
-        for (int base = 0; base < a.p.n_chunks; base += 2 * kCtas) {
-            const int ch = base + 2 * cta + half;
-            const bool has = ch < a.p.n_chunks;
-            int cnt = 0, c = 0;
-            if (has) {
-                const int p0 = __ldg(a.p.chunk_p0 + ch);
-                cnt = __ldg(a.p.chunk_p1 + ch) - p0;
-                c = __ldg(a.p.chunk_tile + ch) * kTileCols + lane * 4;
-                for (int t = ht; t < cnt; t += kBlk) {
-                    if (loops == 0 || a.p.n_chunks > 2 * kCtas) {  // one round: the chunk's rows stay in place
-                        const int4 dd = __ldg(a.p.trow_desc + p0 + t);
-                        s.cl[half][t] = make_int2(dd.x, dd.y);
-                        s.off[half][t] = __ldg(a.p.trow_off + p0 + t);
-                        s.slot[half][t] = dd.z;
-                    }
-                    const double* y = a.p.ypart + 3 * (size_t)s.slot[half][t];
-#pragma unroll
-                    for (int d = 0; d < 3; ++d) s.y[half][d][t] = __ldcg(y + d);
+        // ---- S^T chunks: one per CTA (k_spmv_ST_part's order) ----
+        for (int ch = cta; ch < a.p.n_chunks; ch += kCtas) {
+            const int p0 = __ldg(a.p.chunk_p0 + ch), cnt = __ldg(a.p.chunk_p1 + ch) - p0;
+            const int c = __ldg(a.p.chunk_tile + ch) * kTileCols + lane * 4;
+            for (int t = tid; t < cnt; t += kThr) {
+                if (loops == 0 || a.p.n_chunks > kCtas) {  // one chunk a CTA: its rows stay in place
+                    const int4 dd = __ldg(a.p.trow_desc + p0 + t);
+                    s.cl[t] = make_int2(dd.x, dd.y);
+                    s.off[t] = __ldg(a.p.trow_off + p0 + t);
+                    s.slot[t] = dd.z;
                 }
+                const double* y = a.p.ypart + 3 * (size_t)s.slot[t];
+#pragma unroll
+                for (int d = 0; d < 3; ++d) s.y[d][t] = __ldcg(y + d);
             }
             __syncthreads();
             double acc[3][4];
@@ -265,7 +258,7 @@ __global__ void __launch_bounds__(kThr, 1) k_small_loop(SmallLoop a, int cap) {
             for (int d = 0; d < 3; ++d)
 #pragma unroll
                 for (int q = 0; q < 4; ++q) acc[d][q] = 0.0;
-            for (int b = hw; b < cnt; b += 32) {
+            for (int b = wid; b < cnt; b += 32) {
                 double sv[4][4];
                 bool in[4];
 #pragma unroll
@@ -273,10 +266,10 @@ __global__ void __launch_bounds__(kThr, 1) k_small_loop(SmallLoop a, int cap) {
                     const int t = b + 8 * u;
                     in[u] = false;
                     if (t < cnt) {
-                        const int2 cl = s.cl[half][t];
+                        const int2 cl = s.cl[t];
                         in[u] = cl.y > 0 && c >= cl.x && c + 4 <= cl.x + cl.y;
                         if (in[u]) {
-                            const double2* q = reinterpret_cast<const double2*>(a.p.vals + s.off[half][t] + (c - cl.x));
+                            const double2* q = reinterpret_cast<const double2*>(a.p.vals + s.off[t] + (c - cl.x));
                             const double2 x0 = __ldg(q), x1 = __ldg(q + 1);
                             sv[u][0] = x0.x; sv[u][1] = x0.y; sv[u][2] = x1.x; sv[u][3] = x1.y;
                         }
@@ -286,7 +279,7 @@ __global__ void __launch_bounds__(kThr, 1) k_small_loop(SmallLoop a, int cap) {
                 for (int u = 0; u < 4; ++u)
                     if (in[u]) {
                         const int t = b + 8 * u;
-                        const double y0 = s.y[half][0][t], y1 = s.y[half][1][t], y2 = s.y[half][2][t];
+                        const double y0 = s.y[0][t], y1 = s.y[1][t], y2 = s.y[2][t];
 #pragma unroll
                         for (int q = 0; q < 4; ++q) {
                             acc[0][q] += sv[u][q] * y0;
@@ -298,16 +291,15 @@ __global__ void __launch_bounds__(kThr, 1) k_small_loop(SmallLoop a, int cap) {
 #pragma unroll
             for (int d = 0; d < 3; ++d)
 #pragma unroll
-                for (int q = 0; q < 4; ++q) s.red[half][hw][d][lane * 4 + q] = acc[d][q];
+                for (int q = 0; q < 4; ++q) s.red[wid][d][lane * 4 + q] = acc[d][q];
             __syncthreads();
-            if (has)
-                for (int t = ht; t < 3 * kTileCols; t += kBlk) {
-                    const int d = t / kTileCols, cc = t % kTileCols;
-                    double sum = 0.0;
+            for (int t = tid; t < 3 * kTileCols; t += kThr) {
+                const int d = t / kTileCols, cc = t % kTileCols;
+                double sum = 0.0;
 #pragma unroll
-                    for (int w = 0; w < 8; ++w) sum += s.red[half][w][d][cc];
-                    a.p.xpart[(size_t)ch * 3 * kTileCols + t] = sum;
-                }
+                for (int w = 0; w < 8; ++w) sum += s.red[w][d][cc];
+                a.p.xpart[(size_t)ch * 3 * kTileCols + t] = sum;
+            }
             __syncthreads();
         }
         cluster_sync();
@@ -331,38 +323,33 @@ __global__ void __launch_bounds__(kThr, 1) k_small_loop(SmallLoop a, int cap) {
                 if (count >= 1) {
                     const int sl = (head + count - 1) % W;
                     gnew = g - lg;
-                    s.hist[sl][ht] = gnew;
-                    s.hist[kMaxWindow + sl][ht] = xp - lx;
+                    s.hist[sl][tid] = gnew;
+                    s.hist[kMaxWindow + sl][tid] = xp - lx;
                 }
                 lg = g;
                 lx = xp;
             }
         }
         if (cta < nblk) {
-            if (half == 0) {
 #pragma unroll 1
-                for (int j = 0; j < m; ++j) {
-                    const double dgj = own ? s.hist[(head + j) % W][ht] : 0.0;
-                    const double t0 = wsum(gnew * dgj), t1 = wsum(dgj * g);
-                    if (lane == 0) {
-                        s.sh[j][wid] = t0;
-                        s.sh[m + j][wid] = t1;
-                    }
-                }
-                const double t0 = wsum(g * g), t1 = wsum(xv * xv);
+            for (int j = 0; j < m; ++j) {
+                const double dgj = own ? s.hist[(head + j) % W][tid] : 0.0;
+                const double t0 = wsum(gnew * dgj), t1 = wsum(dgj * g);
                 if (lane == 0) {
-                    s.sh[2 * m][wid] = t0;
-                    s.sh[2 * m + 1][wid] = t1;
+                    s.sh[j][wid] = t0;
+                    s.sh[m + j][wid] = t1;
                 }
+            }
+            const double t0 = wsum(g * g), t1 = wsum(xv * xv);
+            if (lane == 0) {
+                s.sh[2 * m][wid] = t0;
+                s.sh[2 * m + 1][wid] = t1;
             }
             __syncthreads();
-            if (wid < nv) {
-                const double t = wsum(lane < kBlk / 32 ? s.sh[wid][lane] : 0.0);
-                if (lane == 0) a.part_aa[(size_t)cta * kAaVals + wid] = t;
-            }
-            if (wid + 16 < nv) {  // window 8: 18 values, 16 warps
-                const double t = wsum(lane < kBlk / 32 ? s.sh[wid + 16][lane] : 0.0);
-                if (lane == 0) a.part_aa[(size_t)cta * kAaVals + wid + 16] = t;
+#pragma unroll 1
+            for (int i = wid; i < nv; i += kThr / 32) {
+                const double t = wsum(lane < kThr / 32 ? s.sh[i][lane] : 0.0);
+                if (lane == 0) a.part_aa[(size_t)cta * kAaVals + i] = t;
             }
         }
         cluster_sync();
@@ -394,7 +381,7 @@ __global__ void __launch_bounds__(kThr, 1) k_small_loop(SmallLoop a, int cap) {
 #pragma unroll 1
                 for (int j = 0; j < m; ++j) {
                     const int sl = (head + j) % W;
-                    xn -= (s.hist[kMaxWindow + sl][ht] + s.hist[sl][ht]) * s.aa.gamma[j];
+                    xn -= (s.hist[kMaxWindow + sl][tid] + s.hist[sl][tid]) * s.aa.gamma[j];
                 }
                 if (fx) xn = fv;
             }
@@ -405,16 +392,14 @@ __global__ void __launch_bounds__(kThr, 1) k_small_loop(SmallLoop a, int cap) {
             xp = xn;
         }
         if (cta < nblk) {
-            if (half == 0) {
 #pragma unroll
-                for (int i = 0; i < 3; ++i) {
-                    const double t = wsum(u3[i]);
-                    if (lane == 0) s.sh[i][wid] = t;
-                }
+            for (int i = 0; i < 3; ++i) {
+                const double t = wsum(u3[i]);
+                if (lane == 0) s.sh[i][wid] = t;
             }
             __syncthreads();
             if (wid < 3) {
-                const double t = wsum(lane < kBlk / 32 ? s.sh[wid][lane] : 0.0);
+                const double t = wsum(lane < kThr / 32 ? s.sh[wid][lane] : 0.0);
                 if (lane == 0) a.part_upd[3 * cta + wid] = t;
             }
         }
