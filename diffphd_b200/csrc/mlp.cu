@@ -1,15 +1,15 @@
 // Learned warm start of the PD fixed point: a per-node MLP 15 -> 128 -> 128 -> 3 (GELU), BF16 weights and
 // activations on the tensor cores (mma.sync m16n8k16, FP32 accumulation), FP32 master weights and AdamW.
 //
-// Layout.  Rows are nodes (one sample = one node at one time step).  Every warp owns 16 rows; a CTA of 8
-// warps owns 128 rows.  The three layers are chained in registers: the FP32 accumulator fragment of one layer
-// is the BF16 A-operand fragment of the next (columns 16kk..16kk+15 of the next layer's K are the n-tiles
+// Layout.  Rows are nodes (one sample = one node at one time step); a CTA owns 128 rows, in groups of 16.  In
+// k_mlp_forward a warp owns a group and the three layers are chained in registers: the FP32 accumulator fragment of one
+// layer is the BF16 A-operand fragment of the next (columns 16kk..16kk+15 of the next layer's K are the n-tiles
 // 2kk, 2kk+1 of the previous layer's output).  Weight matrices live in shared memory in the "col" layout the
 // B operand wants (W^T, i.e. [out][in] with `in` contiguous).
 //
-// Training step (k_mlp_train): forward with the activations kept in registers, backward through the same
-// fragments, then the CTA's rows are staged in shared memory and its weight-gradient partials
-// (x^T dz1, a1^T dz2, a2^T dz3) are formed by tensor-core MMAs over the 128 rows; k_mlp_adamw sums the CTA
+// Training step (k_mlp_train): two warps share a group; each layer's rows are staged in shared memory, where the next
+// one and the weight-gradient partials (x^T dz1, a1^T dz2, a2^T dz3: tensor-core MMAs over the 128 rows) read
+// them; k_mlp_adamw sums the CTA
 // partials in a fixed order (deterministic), applies AdamW to the FP32 master weights and re-packs the BF16
 // copies.  Features are built on the device by k_mlp_features.
 #include <cuda_bf16.h>
@@ -148,17 +148,19 @@ __device__ __forceinline__ void load_x(const __nv_bfloat16* X, int r0, int n, ui
     a[3] = rb < n ? ld32(X + (size_t)rb * kIn + 2 * t + 8) : 0u;
 }
 
-// Layer 1 pre-activations (16 x 128) for one warp.
-__device__ __forceinline__ void layer1(const Smem& s, const uint32_t* ax, float (*z)[4]) {
+// Layer 1 pre-activations (16 rows, NJ 8-column tiles from tile j0) for one warp.
+template <int NJ>
+__device__ __forceinline__ void layer1(const Smem& s, const uint32_t* ax, float (*z)[4], int j0) {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
+    for (int jj = 0; jj < NJ; ++jj) {
+        const int j = j0 + jj;
         const uint32_t b[2] = {ld32(&s.W1T[(8 * j + g) * kIn + 2 * t]), ld32(&s.W1T[(8 * j + g) * kIn + 2 * t + 8])};
-        z[j][0] = s.b1[8 * j + 2 * t];
-        z[j][1] = s.b1[8 * j + 2 * t + 1];
-        z[j][2] = z[j][0];
-        z[j][3] = z[j][1];
-        mma16816(z[j], ax, b);
+        z[jj][0] = s.b1[8 * j + 2 * t];
+        z[jj][1] = s.b1[8 * j + 2 * t + 1];
+        z[jj][2] = z[jj][0];
+        z[jj][3] = z[jj][1];
+        mma16816(z[jj], ax, b);
     }
 }
 
@@ -197,7 +199,42 @@ __device__ __forceinline__ void layer_hh(const __nv_bfloat16* BT, const float* b
         }
 }
 
-__device__ __forceinline__ void layer3(const Smem& s, uint32_t (*a)[4], float* c) {
+// A fragment (16 rows from r0, k-step kk) of a swizzled row tile.
+__device__ __forceinline__ void ld_afrag(const __nv_bfloat16* tile, int r0, int kk, uint32_t* a) {
+    const int lane = threadIdx.x & 31, mat = lane >> 3, mr = lane & 7;
+    ldsm4(tile + swz(r0 + (mat & 1) * 8 + mr, 16 * kk + (mat >> 1) * 8), a);
+}
+
+// layer_hh with A from a swizzled row tile (rows r0..r0+15), for the eight 8-column tiles from j0.
+__device__ __forceinline__ void layer_tile(const __nv_bfloat16* BT, const float* bias, const __nv_bfloat16* rows, int r0,
+                                           int j0, float (*c)[4]) {
+    const int lane = threadIdx.x & 31, t = lane & 3;
+    const int mat = lane >> 3, mr = lane & 7;
+#pragma unroll
+    for (int jj = 0; jj < 8; ++jj) {
+        c[jj][0] = bias ? bias[8 * (j0 + jj) + 2 * t] : 0.f;
+        c[jj][1] = bias ? bias[8 * (j0 + jj) + 2 * t + 1] : 0.f;
+        c[jj][2] = c[jj][0];
+        c[jj][3] = c[jj][1];
+    }
+#pragma unroll 2  // fully unrolled, the hoisted loads spill
+    for (int kk = 0; kk < 8; kk += 2) {
+        uint32_t a[2][4];
+        ld_afrag(rows, r0, kk, a[0]);
+        ld_afrag(rows, r0, kk + 1, a[1]);
+#pragma unroll
+        for (int jj = 0; jj < 8; ++jj) {
+            uint32_t b[4];  // two k-steps
+            ldsm4(BT + swz(8 * (j0 + jj) + mr, 16 * kk + 8 * mat), b);
+            mma16816(c[jj], a[0], b);
+            mma16816(c[jj], a[1], b + 2);
+        }
+    }
+}
+
+// Output layer of one warp's 16 rows; afrag(kk, a): the A fragment of k-step kk.
+template <class AFrag>
+__device__ __forceinline__ void layer3(const Smem& s, AFrag afrag, float* c) {
     const int lane = threadIdx.x & 31, t = lane & 3;
     const int mat = lane >> 3, mr = lane & 7;
     c[0] = s.b3[2 * t];
@@ -206,10 +243,12 @@ __device__ __forceinline__ void layer3(const Smem& s, uint32_t (*a)[4], float* c
     c[3] = c[1];
 #pragma unroll
     for (int kk = 0; kk < 8; kk += 2) {
-        uint32_t b[4];
+        uint32_t b[4], a[2][4];
+        afrag(kk, a[0]);
+        afrag(kk + 1, a[1]);
         ldsm4(s.W3T + swz(mr, 16 * kk + 8 * mat), b);
-        mma16816(c, a[kk], b);
-        mma16816(c, a[kk + 1], b + 2);
+        mma16816(c, a[0], b);
+        mma16816(c, a[1], b + 2);
     }
 }
 
@@ -225,7 +264,7 @@ __global__ void __launch_bounds__(256) k_mlp_forward(MlpParams p, const __nv_bfl
     uint32_t ax[4];
     load_x(X, r0, n, ax);
     float z[16][4];
-    layer1(s, ax, z);
+    layer1<16>(s, ax, z, 0);
 #pragma unroll
     for (int j = 0; j < 16; ++j)
 #pragma unroll
@@ -239,7 +278,9 @@ __global__ void __launch_bounds__(256) k_mlp_forward(MlpParams p, const __nv_bfl
         for (int e = 0; e < 4; ++e) z[j][e] = gelu(z[j][e]);
     to_afrag(z, a);
     float o[4];
-    layer3(s, a, o);
+    layer3(s, [&](int kk, uint32_t* f) {
+        for (int e = 0; e < 4; ++e) f[e] = a[kk][e];
+    }, o);
     const int ra = r0 + g, rb = r0 + g + 8;
     if (ra < n) { out[(size_t)ra * kOut + 2 * t] = o[0]; out[(size_t)ra * kOut + 2 * t + 1] = o[1]; }
     if (rb < n) { out[(size_t)rb * kOut + 2 * t] = o[2]; out[(size_t)rb * kOut + 2 * t + 1] = o[3]; }
@@ -257,9 +298,14 @@ __device__ __forceinline__ void colsum(const float* c, float& s0, float& s1) {
 }
 
 // One training step over rows [128*blockIdx, +128): MSE(out[:, :3], Y) / n_total, per-CTA gradient partials.
-__global__ void __launch_bounds__(256) k_mlp_train(MlpParams p, const __nv_bfloat16* __restrict__ X,
-                                                   const float* __restrict__ Y, int n, float inv_n,
-                                                   float* __restrict__ part) {
+// Bound by the erf / exp arithmetic of the activations and its latency; the staged rows and both weight orders fill the
+// SM's shared memory, so one CTA an SM.  Two warps share 16 rows, each with half of every layer's columns, and hand the
+// halves over through the staged row tiles: sixteen warps hide what eight (one per 16 rows, activations chained in
+// registers) left exposed.  A step on 65,536 rows (this kernel and the AdamW one): 157 us with eight, 116 with sixteen.
+constexpr int kTrainThreads = 512;
+__global__ void __launch_bounds__(kTrainThreads) k_mlp_train(MlpParams p, const __nv_bfloat16* __restrict__ X,
+                                                             const float* __restrict__ Y, int n, float inv_n,
+                                                             float* __restrict__ part) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SmemTrain& s = *reinterpret_cast<SmemTrain*>(smem_raw);
     load_weights(s.f, p);
@@ -267,19 +313,16 @@ __global__ void __launch_bounds__(256) k_mlp_train(MlpParams p, const __nv_bfloa
     copy_plain(s.W3b, p.W3b, kHid * 16);
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int rl = warp * 16;  // local row base
+    const int rw = warp & 7, half = warp >> 3, j0 = 8 * half;  // 16-row group, column half, its first 8-column tile
+    const int rl = rw * 16;                                    // local row base
     const int r0 = blockIdx.x * kRowsPerCta + rl;
-    // Rows of the warp's tiles are staged in shared memory as soon as they are final (A-fragment order back
-    // to row-major), so that only the packed GELU derivatives stay live across the backward pass.
+    // the two warps of a row group have written their halves of a row tile
+    auto pair_sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(1 + rw) : "memory"); };
     auto put = [&](__nv_bfloat16* at, uint32_t v) { *reinterpret_cast<uint32_t*>(at) = v; };
-    auto stage = [&](__nv_bfloat16* dst, const uint32_t (*fr)[4]) {  // 128 columns
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-            put(dst + swz(rl + g, 16 * kk + 2 * t), fr[kk][0]);
-            put(dst + swz(rl + g + 8, 16 * kk + 2 * t), fr[kk][1]);
-            put(dst + swz(rl + g, 16 * kk + 2 * t + 8), fr[kk][2]);
-            put(dst + swz(rl + g + 8, 16 * kk + 2 * t + 8), fr[kk][3]);
-        }
+    // one 8-column accumulator tile of the warp's rows, as BF16
+    auto stage = [&](__nv_bfloat16* dst, int j, uint32_t lo, uint32_t hi) {
+        put(dst + swz(rl + g, 8 * j + 2 * t), lo);
+        put(dst + swz(rl + g + 8, 8 * j + 2 * t), hi);
     };
     auto stage16 = [&](__nv_bfloat16* dst, const uint32_t* fr) {  // 16 columns
         put(dst + (rl + g) * 16 + 2 * t, fr[0]);
@@ -287,38 +330,28 @@ __global__ void __launch_bounds__(256) k_mlp_train(MlpParams p, const __nv_bfloa
         put(dst + (rl + g) * 16 + 2 * t + 8, fr[2]);
         put(dst + (rl + g + 8) * 16 + 2 * t + 8, fr[3]);
     };
-    // ---- forward ----
-    uint32_t ax[1][4];
-    load_x(X, r0, n, ax[0]);
-    stage16(s.x, ax[0]);
-    float c[16][4];
-    layer1(s.f, ax[0], c);  // z1
-    // gelu'(z1) and gelu'(z2) are parked (BF16, accumulator order) in the dz1 / dz2 tiles, which each thread
-    // later overwrites at the same positions with its own dz values
-    auto park = [&](__nv_bfloat16* dst, int j, uint32_t lo, uint32_t hi) {
-        put(dst + swz(rl + g, 8 * j + 2 * t), lo);
-        put(dst + swz(rl + g + 8, 8 * j + 2 * t), hi);
+    // gelu'(z) is parked (BF16) in the tile of dz, which each thread later overwrites at the same positions
+    auto activate = [&](float (*c)[4], __nv_bfloat16* act, __nv_bfloat16* dz) {
+#pragma unroll
+        for (int jj = 0; jj < 8; ++jj) {
+            float* z = c[jj];
+            stage(dz, j0 + jj, pack_bf16(gelu_d(z[0]), gelu_d(z[1])), pack_bf16(gelu_d(z[2]), gelu_d(z[3])));
+            stage(act, j0 + jj, pack_bf16(gelu(z[0]), gelu(z[1])), pack_bf16(gelu(z[2]), gelu(z[3])));
+        }
     };
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-        park(s.dz1, j, pack_bf16(gelu_d(c[j][0]), gelu_d(c[j][1])), pack_bf16(gelu_d(c[j][2]), gelu_d(c[j][3])));
-#pragma unroll
-        for (int e = 0; e < 4; ++e) c[j][e] = gelu(c[j][e]);
-    }
-    uint32_t af[8][4];
-    to_afrag(c, af);  // a1
-    stage(s.a1, af);
-    layer_hh(s.f.W2T, s.f.b2, af, c);  // z2
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-        park(s.dz2, j, pack_bf16(gelu_d(c[j][0]), gelu_d(c[j][1])), pack_bf16(gelu_d(c[j][2]), gelu_d(c[j][3])));
-#pragma unroll
-        for (int e = 0; e < 4; ++e) c[j][e] = gelu(c[j][e]);
-    }
-    to_afrag(c, af);  // a2
-    stage(s.a2, af);
-    float o[4];
-    layer3(s.f, af, o);
+    // ---- forward ----
+    uint32_t ax[4];
+    load_x(X, r0, n, ax);
+    if (half == 0) stage16(s.x, ax);
+    float c[8][4];
+    layer1<8>(s.f, ax, c, j0);  // z1
+    activate(c, s.a1, s.dz1);
+    pair_sync();
+    layer_tile(s.f.W2T, s.f.b2, s.a1, rl, j0, c);  // z2
+    activate(c, s.a2, s.dz2);
+    pair_sync();
+    float o[4];  // both warps of the pair
+    layer3(s.f, [&](int kk, uint32_t* a) { ld_afrag(s.a2, rl, kk, a); }, o);
     // ---- loss gradient dz3 = 2 (pred - y) / n (3 used outputs), and the loss ----
     const int ra = r0 + g, rb = r0 + g + 8;
     float dz3[4] = {0.f, 0.f, 0.f, 0.f}, lsum = 0.f;
@@ -332,59 +365,53 @@ __global__ void __launch_bounds__(256) k_mlp_train(MlpParams p, const __nv_bfloa
         }
     }
     // ---- backward ----
-    const uint32_t adz3[1][4] = {{pack_bf16(dz3[0], dz3[1]), pack_bf16(dz3[2], dz3[3]), 0u, 0u}};
-    stage16(s.dz3, adz3[0]);
+    const uint32_t adz3[4] = {pack_bf16(dz3[0], dz3[1]), pack_bf16(dz3[2], dz3[3]), 0u, 0u};
     float bs[2];
-    colsum(dz3, bs[0], bs[1]);
-    if (lane < 4) {
-        s.red[warp][2 * kHid + 2 * lane] = bs[0];
-        s.red[warp][2 * kHid + 2 * lane + 1] = bs[1];
-    }
-    float ls = lsum;
+    if (half == 0) {
+        stage16(s.dz3, adz3);
+        colsum(dz3, bs[0], bs[1]);
+        if (lane < 4) {
+            s.red[rw][2 * kHid + 2 * lane] = bs[0];
+            s.red[rw][2 * kHid + 2 * lane + 1] = bs[1];
+        }
+        float ls = lsum;
 #pragma unroll
-    for (int of = 16; of > 0; of >>= 1) ls += __shfl_xor_sync(0xffffffffu, ls, of);
-    if (lane == 0) s.red[warp][2 * kHid + kOut] = ls;
-    auto unpack_mul = [&](float* cj, const __nv_bfloat16* src, int j) {
-        const float2 lo =
-            __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(src + swz(rl + g, 8 * j + 2 * t)));
+        for (int of = 16; of > 0; of >>= 1) ls += __shfl_xor_sync(0xffffffffu, ls, of);
+        if (lane == 0) s.red[rw][2 * kHid + kOut] = ls;
+    }
+    // times the parked gelu', column sums for the bias gradient, and the tile itself
+    auto finish = [&](float* cj, __nv_bfloat16* dz, int j, int red0) {
+        const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(dz + swz(rl + g, 8 * j + 2 * t)));
         const float2 hi =
-            __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(src + swz(rl + g + 8, 8 * j + 2 * t)));
+            __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(dz + swz(rl + g + 8, 8 * j + 2 * t)));
         cj[0] *= lo.x;
         cj[1] *= lo.y;
         cj[2] *= hi.x;
         cj[3] *= hi.y;
+        colsum(cj, bs[0], bs[1]);
+        if (lane < 4) {
+            s.red[rw][red0 + 8 * j + 2 * lane] = bs[0];
+            s.red[rw][red0 + 8 * j + 2 * lane + 1] = bs[1];
+        }
+        stage(dz, j, pack_bf16(cj[0], cj[1]), pack_bf16(cj[2], cj[3]));
     };
     // da2 = dz3 W3^T  (K = outputs padded to 16); dz2 = da2 * gelu'(z2)
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-        c[j][0] = c[j][1] = c[j][2] = c[j][3] = 0.f;
+    for (int jj = 0; jj < 8; ++jj) {
+        const int j = j0 + jj;
+        c[jj][0] = c[jj][1] = c[jj][2] = c[jj][3] = 0.f;
         const uint32_t b[2] = {ld32(&s.W3b[(8 * j + g) * 16 + 2 * t]), ld32(&s.W3b[(8 * j + g) * 16 + 2 * t + 8])};
-        mma16816(c[j], adz3[0], b);
-        unpack_mul(c[j], s.dz2, j);
-        colsum(c[j], bs[0], bs[1]);
-        if (lane < 4) {
-            s.red[warp][kHid + 8 * j + 2 * lane] = bs[0];
-            s.red[warp][kHid + 8 * j + 2 * lane + 1] = bs[1];
-        }
+        mma16816(c[jj], adz3, b);
+        finish(c[jj], s.dz2, j, kHid);
     }
-    to_afrag(c, af);  // dz2
-    stage(s.dz2, af);
+    pair_sync();
     // da1 = dz2 W2^T, B from W2b ([in][out]); dz1 = da1 * gelu'(z1)
-    layer_hh(s.W2b, nullptr, af, c);
+    layer_tile(s.W2b, nullptr, s.dz2, rl, j0, c);
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-        unpack_mul(c[j], s.dz1, j);
-        colsum(c[j], bs[0], bs[1]);
-        if (lane < 4) {
-            s.red[warp][8 * j + 2 * lane] = bs[0];
-            s.red[warp][8 * j + 2 * lane + 1] = bs[1];
-        }
-    }
-    to_afrag(c, af);  // dz1
-    stage(s.dz1, af);
+    for (int jj = 0; jj < 8; ++jj) finish(c[jj], s.dz1, j0 + jj, 0);
     __syncthreads();
     float* P = part + (size_t)blockIdx.x * kPartSize;
-    // biases and loss (fixed warp order)
+    // biases and loss (fixed order of the row groups)
     for (int i = threadIdx.x; i < 2 * kHid + kOut + 1; i += blockDim.x) {
         float v = 0.f;
         for (int w = 0; w < 8; ++w) v += s.red[w][i];
@@ -405,12 +432,12 @@ __global__ void __launch_bounds__(256) k_mlp_train(MlpParams p, const __nv_bfloa
         dst[(m0 + g + 8) * ld + n0 + 2 * t + 1] = acc[3];
     };
     uint32_t A[kSteps][4];
-    // dW2 [in][out] = a1^T dz2: warp owns input rows [16w, 16w+16)
+    // dW2 [in][out] = a1^T dz2: warp owns input rows [16 rw, 16 rw + 16) and its half of the columns
 #pragma unroll
     for (int kk = 0; kk < kSteps; ++kk)
-        ldsm4t(s.a1 + swz(16 * kk + (mat >> 1) * 8 + mr, 16 * warp + (mat & 1) * 8), A[kk]);
+        ldsm4t(s.a1 + swz(16 * kk + (mat >> 1) * 8 + mr, 16 * rw + (mat & 1) * 8), A[kk]);
 #pragma unroll 2
-    for (int j = 0; j < 16; j += 2) {
+    for (int j = j0; j < j0 + 8; j += 2) {
         float acc[2][4] = {};
 #pragma unroll
         for (int kk = 0; kk < kSteps; ++kk) {
@@ -419,34 +446,33 @@ __global__ void __launch_bounds__(256) k_mlp_train(MlpParams p, const __nv_bfloa
             mma16816(acc[0], A[kk], B);
             mma16816(acc[1], A[kk], B + 2);
         }
-        store(P + kPartW2, kHid, 16 * warp, 8 * j, acc[0]);
-        store(P + kPartW2, kHid, 16 * warp, 8 * (j + 1), acc[1]);
+        store(P + kPartW2, kHid, 16 * rw, 8 * j, acc[0]);
+        store(P + kPartW2, kHid, 16 * rw, 8 * (j + 1), acc[1]);
     }
-    // dW3 [hidden][out=8] = a2^T dz3: warp owns hidden rows [16w, 16w+16)
-    {
+    if (half == 0) {
+        // dW3 [hidden][out=8] = a2^T dz3: warp owns hidden rows [16 rw, 16 rw + 16)
         float acc[4] = {};
 #pragma unroll
         for (int kk = 0; kk < kSteps; ++kk) {
             uint32_t B[2];
-            ldsm4t(s.a2 + swz(16 * kk + (mat >> 1) * 8 + mr, 16 * warp + (mat & 1) * 8), A[kk]);
+            ldsm4t(s.a2 + swz(16 * kk + (mat >> 1) * 8 + mr, 16 * rw + (mat & 1) * 8), A[kk]);
             ldsm2t(s.dz3 + (16 * kk + (mat & 1) * 8 + mr) * 16, B);
             mma16816(acc, A[kk], B);
         }
-        store(P + kPartW3, kOut, 16 * warp, 0, acc);
-    }
-    // dW1 [in=16][out] = x^T dz1: warp owns output n-tiles 2w, 2w+1
-    {
+        store(P + kPartW3, kOut, 16 * rw, 0, acc);
+    } else {
+        // dW1 [in=16][out] = x^T dz1: warp owns output n-tiles 2 rw, 2 rw + 1
         float acc[2][4] = {};
 #pragma unroll
         for (int kk = 0; kk < kSteps; ++kk) {
             uint32_t B[4];
             ldsm4t(s.x + (16 * kk + (mat >> 1) * 8 + mr) * 16 + (mat & 1) * 8, A[kk]);
-            ldsm4t(s.dz1 + swz(16 * kk + (mat & 1) * 8 + mr, 8 * (2 * warp + (mat >> 1))), B);
+            ldsm4t(s.dz1 + swz(16 * kk + (mat & 1) * 8 + mr, 8 * (2 * rw + (mat >> 1))), B);
             mma16816(acc[0], A[kk], B);
             mma16816(acc[1], A[kk], B + 2);
         }
-        store(P + kPartW1, kHid, 0, 8 * (2 * warp), acc[0]);
-        store(P + kPartW1, kHid, 0, 8 * (2 * warp + 1), acc[1]);
+        store(P + kPartW1, kHid, 0, 8 * (2 * rw), acc[0]);
+        store(P + kPartW1, kHid, 0, 8 * (2 * rw + 1), acc[1]);
     }
 }
 
@@ -568,8 +594,8 @@ int launch_mlp_train(const MlpParams& p, const void* X, const float* Y, int n, f
     cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemTrain));
     const int blocks = (n + kRowsPerCta - 1) / kRowsPerCta;
     if (blocks > 0)
-        k_mlp_train<<<blocks, 256, sizeof(SmemTrain), st>>>(p, reinterpret_cast<const __nv_bfloat16*>(X), Y, n,
-                                                             1.f / (float)n, part);
+        k_mlp_train<<<blocks, kTrainThreads, sizeof(SmemTrain), st>>>(p, reinterpret_cast<const __nv_bfloat16*>(X), Y, n,
+                                                                       1.f / (float)n, part);
     return blocks;
 }
 
