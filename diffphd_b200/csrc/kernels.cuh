@@ -126,11 +126,16 @@ struct SpmvPlan {
 // Schedule by the factor's size (padded values).  Long segments and chunks keep more bytes in flight per warp and CTA
 // and leave fewer partial sums; short ones make enough of them to fill the GPU.  Pair times in us, FP64 / FP32:
 //   54 M (48x24x24 hexes)           segment 1,024: 177 / 100   2,048: 167 / 95      4,096: 169 / 98
-//                                   chunk 64: 223 / 107        192: 210 / 99        512: 213 / 105
+//                                   chunk 64: 186 / 99         192: 169 / 93        256: 168 / 94
+//   19 M (24^3 hexes)               chunk 64: 76 / 44          192: 70 / 44         256: 74 / 41
+//   113 M (48x32x28 hexes)          chunk 96: - / 191          192: 339 / 185       256: 338 / 186
 //   224 M (64x32x32 hexes)          segment 2,048: 624 / 338   4,096: 602 / 324     8,192: 601 / 336
 //                                   chunk 64: 903 / 396        192: 827 / 353       512: 812 / 345
 // At 7.3 M (32x16x16 tets) 1,024-column segments would save 5% of the pair, but the sums' order is part of what a
-// contact-free FP64 rollout that stops at a loose gate returns, and there it stays as it is.
+// contact-free FP64 rollout that stops at a loose gate returns, and there it stays as it is.  192 and 256 rows time alike;
+// 256 is taken because of the rotated 24^3 drop with friction, which has a frame with several fixed points within the
+// gate: the sums' rounding decides which one is found, and with 256 rows (as with 96 or 160) it is the one that the CPU
+// solver finds.
 struct StsSizes {
     int seg_cols;    // columns per S v work item
     int chunk_rows;  // rows per S^T chunk CTA
@@ -138,7 +143,7 @@ struct StsSizes {
 };
 constexpr StsSizes sts_sizes(long long values) {
     return values <= (16ll << 20)    ? StsSizes{2048, 64, 4}
-           : values <= (128ll << 20) ? StsSizes{2048, 192, 4}
+           : values <= (128ll << 20) ? StsSizes{2048, 256, 4}
                                      : StsSizes{4096, 512, 8};
 }
 constexpr int kUnitRows = 8;  // rows per S v unit (the row-group cap of the item schedule)

@@ -171,10 +171,10 @@ long long dphd_s_nnz(const dphd_deformable* h);
 /* Stored S values including the 16-byte alignment padding of each row segment. */
 long long dphd_s_padded_values(const dphd_deformable* h);
 
-/* Selects the kernel of the FP32 y = S v pass: 1 one warp per row group of up to 8 rows that share a column
- * segment (v read once per group); 0 one warp per row segment.  Both give bit-identical sums; by default the
- * faster one on the factor is chosen by timing both when the factor is built.  Captured iteration graphs are
- * dropped.  No counterpart in the reference (profiling and A/B timing). */
+/* Selects the kernel of the y = S v pass (FP32 and FP64): 1 one warp per four rows of a group of up to 8 that share a
+ * column segment (v read once per four rows); 0 one warp per row segment.  Both give bit-identical sums; by default
+ * the faster one on the factor is chosen by timing both, for each precision, when the factor is built.  Captured
+ * iteration graphs are dropped.  No counterpart in the reference (profiling and A/B timing). */
 int dphd_debug_set_s_kernel(dphd_deformable* h, int row_groups);
 /* Programmatic dependent launch of the kernels inside the iteration graphs (1, the default: each kernel may
  * launch while its predecessor drains and waits for it on the device; 0: plain stream order).  The setting is
