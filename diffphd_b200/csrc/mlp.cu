@@ -15,6 +15,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "kernels.cuh"
@@ -297,11 +298,12 @@ __device__ __forceinline__ void colsum(const float* c, float& s0, float& s1) {
     }
 }
 
-// One training step over rows [128*blockIdx, +128): MSE(out[:, :3], Y) / n_total, per-CTA gradient partials.
+// One training step, a tile of 128 rows after another: MSE(out[:, :3], Y) / n_total, a gradient partial per tile.
 // Bound by the erf / exp arithmetic of the activations and its latency; the staged rows and both weight orders fill the
 // SM's shared memory, so one CTA an SM.  Two warps share 16 rows, each with half of every layer's columns, and hand the
 // halves over through the staged row tiles: sixteen warps hide what eight (one per 16 rows, activations chained in
-// registers) left exposed.  A step on 65,536 rows (this kernel and the AdamW one): 157 us with eight, 116 with sixteen.
+// registers) left exposed.  A step on 65,536 rows (this kernel and the AdamW one): 157 us with eight, 116 with sixteen;
+// 104 with one CTA an SM that keeps the weights for all its tiles and loads the next tile's rows ahead.
 constexpr int kTrainThreads = 512;
 __global__ void __launch_bounds__(kTrainThreads) k_mlp_train(MlpParams p, const __nv_bfloat16* __restrict__ X,
                                                              const float* __restrict__ Y, int n, float inv_n,
@@ -315,7 +317,6 @@ __global__ void __launch_bounds__(kTrainThreads) k_mlp_train(MlpParams p, const 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int rw = warp & 7, half = warp >> 3, j0 = 8 * half;  // 16-row group, column half, its first 8-column tile
     const int rl = rw * 16;                                    // local row base
-    const int r0 = blockIdx.x * kRowsPerCta + rl;
     // the two warps of a row group have written their halves of a row tile
     auto pair_sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(1 + rw) : "memory"); };
     auto put = [&](__nv_bfloat16* at, uint32_t v) { *reinterpret_cast<uint32_t*>(at) = v; };
@@ -339,140 +340,147 @@ __global__ void __launch_bounds__(kTrainThreads) k_mlp_train(MlpParams p, const 
             stage(act, j0 + jj, pack_bf16(gelu(z[0]), gelu(z[1])), pack_bf16(gelu(z[2]), gelu(z[3])));
         }
     };
-    // ---- forward ----
+    const int tiles = (n + kRowsPerCta - 1) / kRowsPerCta;
     uint32_t ax[4];
-    load_x(X, r0, n, ax);
-    if (half == 0) stage16(s.x, ax);
-    float c[8][4];
-    layer1<8>(s.f, ax, c, j0);  // z1
-    activate(c, s.a1, s.dz1);
-    pair_sync();
-    layer_tile(s.f.W2T, s.f.b2, s.a1, rl, j0, c);  // z2
-    activate(c, s.a2, s.dz2);
-    pair_sync();
-    float o[4];  // both warps of the pair
-    layer3(s.f, [&](int kk, uint32_t* a) { ld_afrag(s.a2, rl, kk, a); }, o);
-    // ---- loss gradient dz3 = 2 (pred - y) / n (3 used outputs), and the loss ----
-    const int ra = r0 + g, rb = r0 + g + 8;
-    float dz3[4] = {0.f, 0.f, 0.f, 0.f}, lsum = 0.f;
+    load_x(X, blockIdx.x * kRowsPerCta + rl, n, ax);
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int r0 = tile * kRowsPerCta + rl;
+        // ---- forward ----
+        if (half == 0) stage16(s.x, ax);
+        float c[8][4];
+        layer1<8>(s.f, ax, c, j0);  // z1
+        if (tile + (int)gridDim.x < tiles) load_x(X, r0 + (int)gridDim.x * kRowsPerCta, n, ax);  // the next tile's rows
+        activate(c, s.a1, s.dz1);
+        pair_sync();
+        layer_tile(s.f.W2T, s.f.b2, s.a1, rl, j0, c);  // z2
+        activate(c, s.a2, s.dz2);
+        pair_sync();
+        float o[4];  // both warps of the pair
+        layer3(s.f, [&](int kk, uint32_t* a) { ld_afrag(s.a2, rl, kk, a); }, o);
+        // ---- loss gradient dz3 = 2 (pred - y) / n (3 used outputs), and the loss ----
+        const int ra = r0 + g, rb = r0 + g + 8;
+        float dz3[4] = {0.f, 0.f, 0.f, 0.f}, lsum = 0.f;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        const int row = e < 2 ? ra : rb, col = 2 * t + (e & 1);
-        if (row < n && col < kOutUsed) {
-            const float d = o[e] - Y[(size_t)row * kOutUsed + col];
-            dz3[e] = 2.f * d * inv_n;
-            lsum += d * d;
+        for (int e = 0; e < 4; ++e) {
+            const int row = e < 2 ? ra : rb, col = 2 * t + (e & 1);
+            if (row < n && col < kOutUsed) {
+                const float d = o[e] - Y[(size_t)row * kOutUsed + col];
+                dz3[e] = 2.f * d * inv_n;
+                lsum += d * d;
+            }
         }
-    }
-    // ---- backward ----
-    const uint32_t adz3[4] = {pack_bf16(dz3[0], dz3[1]), pack_bf16(dz3[2], dz3[3]), 0u, 0u};
-    float bs[2];
-    if (half == 0) {
-        stage16(s.dz3, adz3);
-        colsum(dz3, bs[0], bs[1]);
-        if (lane < 4) {
-            s.red[rw][2 * kHid + 2 * lane] = bs[0];
-            s.red[rw][2 * kHid + 2 * lane + 1] = bs[1];
+        // ---- backward ----
+        const uint32_t adz3[4] = {pack_bf16(dz3[0], dz3[1]), pack_bf16(dz3[2], dz3[3]), 0u, 0u};
+        float bs[2];
+        if (half == 0) {
+            stage16(s.dz3, adz3);
+            colsum(dz3, bs[0], bs[1]);
+            if (lane < 4) {
+                s.red[rw][2 * kHid + 2 * lane] = bs[0];
+                s.red[rw][2 * kHid + 2 * lane + 1] = bs[1];
+            }
+            float ls = lsum;
+#pragma unroll
+            for (int of = 16; of > 0; of >>= 1) ls += __shfl_xor_sync(0xffffffffu, ls, of);
+            if (lane == 0) s.red[rw][2 * kHid + kOut] = ls;
         }
-        float ls = lsum;
+        // times the parked gelu', column sums for the bias gradient, and the tile itself
+        auto finish = [&](float* cj, __nv_bfloat16* dz, int j, int red0) {
+            const float2 lo =
+                __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(dz + swz(rl + g, 8 * j + 2 * t)));
+            const float2 hi =
+                __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(dz + swz(rl + g + 8, 8 * j + 2 * t)));
+            cj[0] *= lo.x;
+            cj[1] *= lo.y;
+            cj[2] *= hi.x;
+            cj[3] *= hi.y;
+            colsum(cj, bs[0], bs[1]);
+            if (lane < 4) {
+                s.red[rw][red0 + 8 * j + 2 * lane] = bs[0];
+                s.red[rw][red0 + 8 * j + 2 * lane + 1] = bs[1];
+            }
+            stage(dz, j, pack_bf16(cj[0], cj[1]), pack_bf16(cj[2], cj[3]));
+        };
+        // da2 = dz3 W3^T  (K = outputs padded to 16); dz2 = da2 * gelu'(z2)
 #pragma unroll
-        for (int of = 16; of > 0; of >>= 1) ls += __shfl_xor_sync(0xffffffffu, ls, of);
-        if (lane == 0) s.red[rw][2 * kHid + kOut] = ls;
-    }
-    // times the parked gelu', column sums for the bias gradient, and the tile itself
-    auto finish = [&](float* cj, __nv_bfloat16* dz, int j, int red0) {
-        const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(dz + swz(rl + g, 8 * j + 2 * t)));
-        const float2 hi =
-            __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(dz + swz(rl + g + 8, 8 * j + 2 * t)));
-        cj[0] *= lo.x;
-        cj[1] *= lo.y;
-        cj[2] *= hi.x;
-        cj[3] *= hi.y;
-        colsum(cj, bs[0], bs[1]);
-        if (lane < 4) {
-            s.red[rw][red0 + 8 * j + 2 * lane] = bs[0];
-            s.red[rw][red0 + 8 * j + 2 * lane + 1] = bs[1];
+        for (int jj = 0; jj < 8; ++jj) {
+            const int j = j0 + jj;
+            c[jj][0] = c[jj][1] = c[jj][2] = c[jj][3] = 0.f;
+            const uint32_t b[2] = {ld32(&s.W3b[(8 * j + g) * 16 + 2 * t]), ld32(&s.W3b[(8 * j + g) * 16 + 2 * t + 8])};
+            mma16816(c[jj], adz3, b);
+            finish(c[jj], s.dz2, j, kHid);
         }
-        stage(dz, j, pack_bf16(cj[0], cj[1]), pack_bf16(cj[2], cj[3]));
-    };
-    // da2 = dz3 W3^T  (K = outputs padded to 16); dz2 = da2 * gelu'(z2)
+        pair_sync();
+        // da1 = dz2 W2^T, B from W2b ([in][out]); dz1 = da1 * gelu'(z1)
+        layer_tile(s.W2b, nullptr, s.dz2, rl, j0, c);
 #pragma unroll
-    for (int jj = 0; jj < 8; ++jj) {
-        const int j = j0 + jj;
-        c[jj][0] = c[jj][1] = c[jj][2] = c[jj][3] = 0.f;
-        const uint32_t b[2] = {ld32(&s.W3b[(8 * j + g) * 16 + 2 * t]), ld32(&s.W3b[(8 * j + g) * 16 + 2 * t + 8])};
-        mma16816(c[jj], adz3, b);
-        finish(c[jj], s.dz2, j, kHid);
-    }
-    pair_sync();
-    // da1 = dz2 W2^T, B from W2b ([in][out]); dz1 = da1 * gelu'(z1)
-    layer_tile(s.W2b, nullptr, s.dz2, rl, j0, c);
+        for (int jj = 0; jj < 8; ++jj) finish(c[jj], s.dz1, j0 + jj, 0);
+        __syncthreads();
+        float* P = part + (size_t)tile * kPartSize;
+        // biases and loss (fixed order of the row groups)
+        for (int i = threadIdx.x; i < 2 * kHid + kOut + 1; i += blockDim.x) {
+            float v = 0.f;
+            for (int w = 0; w < 8; ++w) v += s.red[w][i];
+            if (i < kHid) P[kPartB1 + i] = v;
+            else if (i < 2 * kHid) P[kPartB2 + i - kHid] = v;
+            else if (i < 2 * kHid + kOut) P[kPartB3 + i - 2 * kHid] = v;
+            else P[kPartLoss] = v;
+        }
+        // ---- weight gradients over the CTA's 128 rows: D[m][n] = sum_r L[r][m] R[r][n] ----
+        // A[m][k] = L[k][m] and B[k][n] = R[k][n] are both transposed loads of row-major tiles; a warp keeps the
+        // fragments of its 16 rows of A over all its column tiles.
+        constexpr int kSteps = kRowsPerCta / 16;
+        const int mat = lane >> 3, mr = lane & 7;
+        auto store = [&](float* dst, int ld, int m0, int n0, const float* acc) {
+            dst[(m0 + g) * ld + n0 + 2 * t] = acc[0];
+            dst[(m0 + g) * ld + n0 + 2 * t + 1] = acc[1];
+            dst[(m0 + g + 8) * ld + n0 + 2 * t] = acc[2];
+            dst[(m0 + g + 8) * ld + n0 + 2 * t + 1] = acc[3];
+        };
+        uint32_t A[kSteps][4];
+        // dW2 [in][out] = a1^T dz2: warp owns input rows [16 rw, 16 rw + 16) and its half of the columns
 #pragma unroll
-    for (int jj = 0; jj < 8; ++jj) finish(c[jj], s.dz1, j0 + jj, 0);
-    __syncthreads();
-    float* P = part + (size_t)blockIdx.x * kPartSize;
-    // biases and loss (fixed order of the row groups)
-    for (int i = threadIdx.x; i < 2 * kHid + kOut + 1; i += blockDim.x) {
-        float v = 0.f;
-        for (int w = 0; w < 8; ++w) v += s.red[w][i];
-        if (i < kHid) P[kPartB1 + i] = v;
-        else if (i < 2 * kHid) P[kPartB2 + i - kHid] = v;
-        else if (i < 2 * kHid + kOut) P[kPartB3 + i - 2 * kHid] = v;
-        else P[kPartLoss] = v;
-    }
-    // ---- weight gradients over the CTA's 128 rows: D[m][n] = sum_r L[r][m] R[r][n] ----
-    // A[m][k] = L[k][m] and B[k][n] = R[k][n] are both transposed loads of row-major tiles; a warp keeps the fragments of
-    // its 16 rows of A over all its column tiles.
-    constexpr int kSteps = kRowsPerCta / 16;
-    const int mat = lane >> 3, mr = lane & 7;
-    auto store = [&](float* dst, int ld, int m0, int n0, const float* acc) {
-        dst[(m0 + g) * ld + n0 + 2 * t] = acc[0];
-        dst[(m0 + g) * ld + n0 + 2 * t + 1] = acc[1];
-        dst[(m0 + g + 8) * ld + n0 + 2 * t] = acc[2];
-        dst[(m0 + g + 8) * ld + n0 + 2 * t + 1] = acc[3];
-    };
-    uint32_t A[kSteps][4];
-    // dW2 [in][out] = a1^T dz2: warp owns input rows [16 rw, 16 rw + 16) and its half of the columns
-#pragma unroll
-    for (int kk = 0; kk < kSteps; ++kk)
-        ldsm4t(s.a1 + swz(16 * kk + (mat >> 1) * 8 + mr, 16 * rw + (mat & 1) * 8), A[kk]);
+        for (int kk = 0; kk < kSteps; ++kk)
+            ldsm4t(s.a1 + swz(16 * kk + (mat >> 1) * 8 + mr, 16 * rw + (mat & 1) * 8), A[kk]);
 #pragma unroll 2
-    for (int j = j0; j < j0 + 8; j += 2) {
-        float acc[2][4] = {};
+        for (int j = j0; j < j0 + 8; j += 2) {
+            float acc[2][4] = {};
 #pragma unroll
-        for (int kk = 0; kk < kSteps; ++kk) {
-            uint32_t B[4];  // two n-tiles
-            ldsm4t(s.dz2 + swz(16 * kk + (mat & 1) * 8 + mr, 8 * (j + (mat >> 1))), B);
-            mma16816(acc[0], A[kk], B);
-            mma16816(acc[1], A[kk], B + 2);
+            for (int kk = 0; kk < kSteps; ++kk) {
+                uint32_t B[4];  // two n-tiles
+                ldsm4t(s.dz2 + swz(16 * kk + (mat & 1) * 8 + mr, 8 * (j + (mat >> 1))), B);
+                mma16816(acc[0], A[kk], B);
+                mma16816(acc[1], A[kk], B + 2);
+            }
+            store(P + kPartW2, kHid, 16 * rw, 8 * j, acc[0]);
+            store(P + kPartW2, kHid, 16 * rw, 8 * (j + 1), acc[1]);
         }
-        store(P + kPartW2, kHid, 16 * rw, 8 * j, acc[0]);
-        store(P + kPartW2, kHid, 16 * rw, 8 * (j + 1), acc[1]);
-    }
-    if (half == 0) {
-        // dW3 [hidden][out=8] = a2^T dz3: warp owns hidden rows [16 rw, 16 rw + 16)
-        float acc[4] = {};
+        if (half == 0) {
+            // dW3 [hidden][out=8] = a2^T dz3: warp owns hidden rows [16 rw, 16 rw + 16)
+            float acc[4] = {};
 #pragma unroll
-        for (int kk = 0; kk < kSteps; ++kk) {
-            uint32_t B[2];
-            ldsm4t(s.a2 + swz(16 * kk + (mat >> 1) * 8 + mr, 16 * rw + (mat & 1) * 8), A[kk]);
-            ldsm2t(s.dz3 + (16 * kk + (mat & 1) * 8 + mr) * 16, B);
-            mma16816(acc, A[kk], B);
-        }
-        store(P + kPartW3, kOut, 16 * rw, 0, acc);
-    } else {
-        // dW1 [in=16][out] = x^T dz1: warp owns output n-tiles 2 rw, 2 rw + 1
-        float acc[2][4] = {};
+            for (int kk = 0; kk < kSteps; ++kk) {
+                uint32_t B[2];
+                ldsm4t(s.a2 + swz(16 * kk + (mat >> 1) * 8 + mr, 16 * rw + (mat & 1) * 8), A[kk]);
+                ldsm2t(s.dz3 + (16 * kk + (mat & 1) * 8 + mr) * 16, B);
+                mma16816(acc, A[kk], B);
+            }
+            store(P + kPartW3, kOut, 16 * rw, 0, acc);
+        } else {
+            // dW1 [in=16][out] = x^T dz1: warp owns output n-tiles 2 rw, 2 rw + 1
+            float acc[2][4] = {};
 #pragma unroll
-        for (int kk = 0; kk < kSteps; ++kk) {
-            uint32_t B[4];
-            ldsm4t(s.x + (16 * kk + (mat >> 1) * 8 + mr) * 16 + (mat & 1) * 8, A[kk]);
-            ldsm4t(s.dz1 + swz(16 * kk + (mat & 1) * 8 + mr, 8 * (2 * rw + (mat >> 1))), B);
-            mma16816(acc[0], A[kk], B);
-            mma16816(acc[1], A[kk], B + 2);
+            for (int kk = 0; kk < kSteps; ++kk) {
+                uint32_t B[4];
+                ldsm4t(s.x + (16 * kk + (mat >> 1) * 8 + mr) * 16 + (mat & 1) * 8, A[kk]);
+                ldsm4t(s.dz1 + swz(16 * kk + (mat & 1) * 8 + mr, 8 * (2 * rw + (mat >> 1))), B);
+                mma16816(acc[0], A[kk], B);
+                mma16816(acc[1], A[kk], B + 2);
+            }
+            store(P + kPartW1, kHid, 0, 8 * (2 * rw), acc[0]);
+            store(P + kPartW1, kHid, 0, 8 * (2 * rw + 1), acc[1]);
         }
-        store(P + kPartW1, kHid, 0, 8 * (2 * rw), acc[0]);
-        store(P + kPartW1, kHid, 0, 8 * (2 * rw + 1), acc[1]);
+        __syncthreads();  // the next tile's rows replace these
     }
 }
 
@@ -594,8 +602,8 @@ int launch_mlp_train(const MlpParams& p, const void* X, const float* Y, int n, f
     cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemTrain));
     const int blocks = (n + kRowsPerCta - 1) / kRowsPerCta;
     if (blocks > 0)
-        k_mlp_train<<<blocks, kTrainThreads, sizeof(SmemTrain), st>>>(p, reinterpret_cast<const __nv_bfloat16*>(X), Y, n,
-                                                                       1.f / (float)n, part);
+        k_mlp_train<<<std::min(blocks, device_sms()), kTrainThreads, sizeof(SmemTrain), st>>>(
+            p, reinterpret_cast<const __nv_bfloat16*>(X), Y, n, 1.f / (float)n, part);
     return blocks;
 }
 
