@@ -349,7 +349,6 @@ __global__ void __launch_bounds__(kTrainThreads) k_mlp_train(MlpParams p, const 
         if (half == 0) stage16(s.x, ax);
         float c[8][4];
         layer1<8>(s.f, ax, c, j0);  // z1
-        if (tile + (int)gridDim.x < tiles) load_x(X, r0 + (int)gridDim.x * kRowsPerCta, n, ax);  // the next tile's rows
         activate(c, s.a1, s.dz1);
         pair_sync();
         layer_tile(s.f.W2T, s.f.b2, s.a1, rl, j0, c);  // z2
@@ -417,6 +416,7 @@ __global__ void __launch_bounds__(kTrainThreads) k_mlp_train(MlpParams p, const 
         for (int jj = 0; jj < 8; ++jj) finish(c[jj], s.dz1, j0 + jj, 0);
         __syncthreads();
         float* P = part + (size_t)tile * kPartSize;
+        if (tile + (int)gridDim.x < tiles) load_x(X, r0 + (int)gridDim.x * kRowsPerCta, n, ax);  // the next tile's rows
         // biases and loss (fixed order of the row groups)
         for (int i = threadIdx.x; i < 2 * kHid + kOut + 1; i += blockDim.x) {
             float v = 0.f;
@@ -484,9 +484,30 @@ __global__ void __launch_bounds__(kTrainThreads) k_mlp_train(MlpParams p, const 
     }
 }
 
+// BF16 operand copies of parameter i (a weight; the biases have none), whose master is w.
+__device__ __forceinline__ void pack_param(const MlpParams& p, int i, float w) {
+    if (i < kPartW2) {  // W1 [in][out] -> W1T [out][in]
+        const int in = i / kHid, o = i % kHid;
+        p.W1T[o * kIn + in] = __float2bfloat16_rn(in < 15 ? w : 0.f);
+    } else if (i < kPartW3) {  // W2 [in][out] -> W2T [out][in] and W2b = W2
+        const int k = i - kPartW2, in = k / kHid, o = k % kHid;
+        const __nv_bfloat16 v = __float2bfloat16_rn(w);
+        p.W2T[o * kHid + in] = v;
+        p.W2b[k] = v;
+    } else if (i < kPartB1) {  // W3 [hidden][out] -> W3T [out][hidden], W3b [hidden][16]
+        const int k = i - kPartW3, h = k / kOut, o = k % kOut;
+        const __nv_bfloat16 v = __float2bfloat16_rn(o < kOutUsed ? w : 0.f);
+        p.W3T[o * kHid + h] = v;
+        p.W3b[h * 16 + o] = v;
+        p.W3b[h * 16 + o + 8] = __float2bfloat16_rn(0.f);
+    }
+}
+
 // Sum of the CTA partials, AdamW on the FP32 masters, BF16 re-pack: a block takes 32 consecutive parameters and its eight
 // warps an eighth of the partials each (in order; the eight sums are added in warp order).  One thread per parameter over
-// all partials took 44 us for 512 of them (42 MB): 78 blocks with a serial chain of additions.
+// all partials took 44 us for 512 of them (42 MB): 78 blocks with a serial chain of additions; this takes 13.  The loss's
+// running sum takes its partials 256 at a time (one chain of loads and additions per 32 was the kernel's longest path)
+// and each parameter's BF16 copies are written here: with both, a step of 65,536 rows went from 104 to 95 us.
 constexpr int kAdamWarps = 8;
 __global__ void __launch_bounds__(32 * kAdamWarps) k_mlp_adamw(MlpParams p, const float* __restrict__ part, int nblocks,
                                                                float lr, float beta1, float beta2, float eps, float wd,
@@ -499,9 +520,23 @@ __global__ void __launch_bounds__(32 * kAdamWarps) k_mlp_adamw(MlpParams p, cons
     if (blockIdx.x == gridDim.x - 1) {  // the loss: one running sum over the partials in order
         if (w != 0 || !loss_out) return;
         float l = 0.f;
-        for (int b = 0; b < nblocks; b += 32) {
-            const float t = b + lane < nblocks ? part[(size_t)(b + lane) * kPartSize + kPartLoss] : 0.f;
-            for (int u = 0; u < min(32, nblocks - b); ++u) l += __shfl_sync(0xffffffffu, t, u);
+        for (int b = 0; b < nblocks; b += 256) {
+            float t[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const int at = b + 32 * k + lane;
+                t[k] = at < nblocks ? part[(size_t)at * kPartSize + kPartLoss] : 0.f;
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const int left = nblocks - b - 32 * k;
+                if (left >= 32) {
+#pragma unroll
+                    for (int u = 0; u < 32; ++u) l += __shfl_sync(0xffffffffu, t[k], u);
+                } else {
+                    for (int u = 0; u < left; ++u) l += __shfl_sync(0xffffffffu, t[k], u);
+                }
+            }
         }
         if (lane == 0) *loss_out = l;
         return;
@@ -552,7 +587,10 @@ __global__ void __launch_bounds__(32 * kAdamWarps) k_mlp_adamw(MlpParams p, cons
         decay = false;
     }
     if (grad_out) grad_out[i] = used ? gsum : 0.f;
-    if (!used || lr == 0.f) return;
+    if (!used || lr == 0.f) {
+        pack_param(p, i, *wp);
+        return;
+    }
     const float b1c = 1.f - powf(beta1, (float)step), b2c = 1.f - powf(beta2, (float)step);
     m[i] = beta1 * m[i] + (1.f - beta1) * gsum;
     v[i] = beta2 * v[i] + (1.f - beta2) * gsum * gsum;
@@ -561,27 +599,14 @@ __global__ void __launch_bounds__(32 * kAdamWarps) k_mlp_adamw(MlpParams p, cons
     if (decay) wv -= lr * wd * wv;
     wv -= lr * mh / (sqrtf(vh) + eps);
     *wp = wv;
+    pack_param(p, i, wv);
 }
 
 __global__ void k_mlp_pack(MlpParams p) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < kIn * kHid) {  // W1 [in][out] -> W1T [out][in]
-        const int in = i / kHid, o = i % kHid;
-        p.W1T[o * kIn + in] = __float2bfloat16_rn(in < 15 ? p.W1[i] : 0.f);
-    }
-    if (i < kHid * kHid) {  // W2 [in][out] -> W2T [out][in] and W2b = W2
-        const int in = i / kHid, o = i % kHid;
-        const __nv_bfloat16 w = __float2bfloat16_rn(p.W2[i]);
-        p.W2T[o * kHid + in] = w;
-        p.W2b[i] = w;
-    }
-    if (i < kHid * kOut) {  // W3 [hidden][out] -> W3T [out][hidden], W3b [hidden][16]
-        const int h = i / kOut, o = i % kOut;
-        const __nv_bfloat16 w = __float2bfloat16_rn(o < kOutUsed ? p.W3[i] : 0.f);
-        p.W3T[o * kHid + h] = w;
-        p.W3b[h * 16 + o] = w;
-        p.W3b[h * 16 + o + 8] = __float2bfloat16_rn(0.f);
-    }
+    if (i < kPartW2) pack_param(p, i, p.W1[i]);
+    else if (i < kPartW3) pack_param(p, i, p.W2[i - kPartW2]);
+    else if (i < kPartB1) pack_param(p, i, p.W3[i - kPartW3]);
 }
 
 }  // namespace
@@ -609,12 +634,11 @@ int launch_mlp_train(const MlpParams& p, const void* X, const float* Y, int n, f
 
 void launch_mlp_adamw(const MlpParams& p, const float* part, int nblocks, float lr, float b1, float b2, float eps,
                       float wd, int step, float* m, float* v, float* grad_out, float* loss_out, cudaStream_t st) {
-    k_mlp_adamw<<<(kPartLoss + 31) / 32 + 1, 32 * kAdamWarps, 0, st>>>(p, part, nblocks, lr, b1, b2, eps, wd, step, m, v, grad_out,
-                                                         loss_out);
-    k_mlp_pack<<<(kHid * kHid + 255) / 256, 256, 0, st>>>(p);
+    k_mlp_adamw<<<(kPartLoss + 31) / 32 + 1, 32 * kAdamWarps, 0, st>>>(p, part, nblocks, lr, b1, b2, eps, wd, step, m, v,
+                                                                       grad_out, loss_out);
 }
 
-void launch_mlp_pack(const MlpParams& p, cudaStream_t st) { k_mlp_pack<<<(kHid * kHid + 255) / 256, 256, 0, st>>>(p); }
+void launch_mlp_pack(const MlpParams& p, cudaStream_t st) { k_mlp_pack<<<(kPartB1 + 255) / 256, 256, 0, st>>>(p); }
 
 int mlp_part_size() { return kPartSize; }
 int mlp_param_count() { return kPartLoss; }
