@@ -505,7 +505,7 @@ __device__ __forceinline__ void pack_param(const MlpParams& p, int i, float w) {
 
 // Sum of the CTA partials, AdamW on the FP32 masters, BF16 re-pack: a block takes 32 consecutive parameters and its eight
 // warps an eighth of the partials each (in order; the eight sums are added in warp order).  One thread per parameter over
-// all partials took 44 us for 512 of them (42 MB): 78 blocks with a serial chain of additions; this takes 13.  The loss's
+// all partials took 44 us for 512 of them (42 MB): 78 blocks with a serial chain of additions.  The loss's
 // running sum takes its partials 256 at a time (one chain of loads and additions per 32 was the kernel's longest path)
 // and each parameter's BF16 copies are written here: with both, a step of 65,536 rows went from 104 to 95 us.
 constexpr int kAdamWarps = 8;
