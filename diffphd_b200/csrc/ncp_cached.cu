@@ -216,6 +216,7 @@ k_ncp_cached_solve(ContactDev c, const double* __restrict__ q0, const double* __
     double* dg = c.pcg + 5 * (size_t)ldx;    // diag(M)
     double* part = c.pcg + 9 * (size_t)ldx;  // per-CTA partial sums (omega_ref and E_ref, kept with the factor,
                                              // at 7 ldx and 8 ldx)
+    double* part_r = part + G;               // those of r.r: no barrier lies between the total of p.w and their stores
     // [0] cached factor valid, [1] its ka, [2] candidates not in its list (this launch), [3] the last CG fell back
     int* flags = c.ncp_flags;
     const bool have = flags[0] != 0;
@@ -362,9 +363,9 @@ k_ncp_cached_solve(ContactDev c, const double* __restrict__ q0, const double* __
                 r[a] = rv;
                 acc += rv * rv;
             }
-            cta_partial(wsum(acc), part);
+            cta_partial(wsum(acc), part_r);
             if (!gsync(c.bar, ctrl)) return;
-            const double rr = grid_total(part);
+            const double rr = grid_total(part_r);
             ++it;
             conv = pw > 0.0 && rr <= c.cg_tol * c.cg_tol * rhs2;
             if (!gsync(c.bar, ctrl)) return;
