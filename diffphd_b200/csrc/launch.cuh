@@ -14,7 +14,8 @@ bool pdl_enabled();  // process-wide switch (set_pdl), read when a kernel is lau
 // at once.  Every such kernel then reads ctrl->done with an ordinary load (ordered after the wait's memory
 // clobber) and branches on it before it touches data a predecessor wrote: loads through the read-only path
 // (ld.global.nc, which the compiler may treat as invariant and move across the wait) stay behind that branch, so
-// none is issued before the wait.
+// none is issued before the wait.  A kernel without that branch (k_noalloc_prepare) reads what a predecessor may have
+// written through pointers that are not __restrict__.
 __device__ __forceinline__ void pdl_enter() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -55,11 +55,14 @@ void* scratch_address() {
 
 // Zeroes the control block, then writes b (node-major, 3n) as the permuted SoA right-hand side with
 // Dirichlet nodes set to zero (the same input the forward step hands to the S^T S pair) and clears the
-// padding columns, all inside the scratch array.
+// padding columns, all inside the scratch array.  A call may follow another one's kernels, which read the array that this
+// one writes, and b may be that call's result (A^-1 A^-1 b): this kernel has no ctrl->done to branch on, so b is not
+// __restrict__ -- its loads are ordinary ones, which the wait's memory clobber keeps behind the wait.  `fixed` and `perm`
+// are written at set-up only.
 template <typename T>
-__global__ void k_noalloc_prepare(int n, int npad, const double* __restrict__ b, const unsigned char* __restrict__ fixed,
+__global__ void k_noalloc_prepare(int n, int npad, const double* b, const unsigned char* __restrict__ fixed,
                                   const int* __restrict__ perm, size_t ctrl_off, size_t v_off) {
-    pdl_enter();  // a call may follow another one's kernels, which read the array this one writes
+    pdl_enter();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < (int)(sizeof(Ctrl) / sizeof(int))) reinterpret_cast<int*>(g_noalloc_scratch + ctrl_off)[t] = 0;
     if (t >= npad) return;
