@@ -206,7 +206,10 @@ k_ncp_cached_solve(ContactDev c, const double* __restrict__ q0, const double* __
     const int ldx = (int)c.kcap;
     if (ka == 0) return;
     if (ka <= kNcpSmall) {  // the same in every CTA: no grid barrier is reached
-        if (bid == 0) small_solve(c, ka, q0, r64, smem);
+        if (bid == 0) {
+            small_solve(c, ka, q0, r64, smem);
+            if (tid == 0) c.ncp_stats[1] += 1;
+        }
         return;
     }
     const int nb = (ka + kT - 1) / kT, ld = nb * kT;
@@ -545,7 +548,7 @@ k_ncp_cached_solve(ContactDev c, const double* __restrict__ q0, const double* __
         if (gt == 0) {
             flags[0] = 1;
             flags[1] = ka;
-            c.ncp_stats[1] += 1;  // refactorisations
+            c.ncp_stats[1] += 1;  // fresh factorisations
         }
     } else if (gt == 0) {
         c.ncp_stats[0] += 1;  // solves by the cached factor

@@ -144,8 +144,9 @@ int dphd_warm_start_state(dphd_deformable* h, double* d_buf, int* valid, int set
 /* The NCP's dense solves since the contact set-up (option ncp_solver 1, the default; ncp_solver 0 factors at
  * every PD iteration as the reference does, forward_gpu.cpp:1238-1240): solves by conjugate gradients
  * preconditioned with the cached factor of an earlier PD iteration's system of the same frame (its active list
- * may differ by a few candidates), fresh factorisations, the CG iterations of all cached solves, and the CG
- * attempts that did not converge and fell back to a factorisation.  Any pointer may be NULL.  No counterpart in
+ * may differ by a few candidates), fresh factorisations (every solve of a small active system among them), the CG
+ * iterations of all cached solves, and the CG attempts that did not converge and fell back to a factorisation.
+ * Every PD iteration with an active candidate counts as one solve.  Any pointer may be NULL.  No counterpart in
  * the reference. */
 int dphd_ncp_solve_stats(dphd_deformable* h, long long* cached, long long* refactors, long long* cg_iters,
                          long long* cg_fallbacks);
