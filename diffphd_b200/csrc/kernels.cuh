@@ -330,8 +330,13 @@ struct ContactDev {
     double* vc = nullptr;            // 3 K: the S-pass input at the candidates after the NCP step (FP64)
 };
 void launch_ncp_cached_solve(const ContactDev& c, const double* q0, const double* r64, Ctrl* ctrl, cudaStream_t st);
-// Active systems of at most this many candidates are solved by one CTA in shared memory (no grid barrier).
-constexpr int kNcpSmall = 64;
+// Active systems of at most this many candidates are solved by one CTA in shared memory (no grid barrier).  A column of
+// its factorisation costs three block barriers, so it grows with the system; the grid's CG stays at about thirty grid
+// barriers.  us per PD iteration of a block of two cell layers at rest (medians over eight allocations), one CTA | grid,
+// without / with friction:
+//   42 active 104 / 111 | 127 / 128      49 active 119 / 125 | 131 / 130      56 active 130 / 137 | 135 / 137
+//   64 active 150 / 156 | 133 / 135
+constexpr int kNcpSmall = 56;
 // The preconditioner of the contact-aware adjoint (contact_precond.cu): the three unit directions of the
 // constraint basis, the parts of one application (stage 0: u = J A^-1 r from y = S r, lam = X^T X u per direction
 // block; stage 1: the S-pass input -J^T lam), and the set-up gather of G_b with an identity X_b.

@@ -35,6 +35,7 @@ constexpr int kNcpMaxListChange = 32;  // larger changes of the active list refa
 constexpr double kOmegaMin = 1e-6;     // |omega| below this: the candidate's row is decoupled (E only)
 constexpr double kEDrift = 0.1;        // |E - (omega / omega_ref)^2 E_ref| above this fraction of M_kk: diagonal
 constexpr long long kSpins = 1ll << 24;
+static_assert(kNcpSmall <= kT, "a small system fits one tile of shared memory");
 
 __device__ __forceinline__ double wsum(double v) { return ncp_warp_sum(v); }
 
@@ -147,7 +148,8 @@ __device__ __forceinline__ void tile_fma(const double* sA, const double* sB, dou
 
 // An active system of at most kNcpSmall candidates, by one CTA: M in shared memory, Cholesky, two triangular solves by
 // one warp, then the multipliers and the cone.  The grid's phases below cost about 5 us per grid barrier (67 us for
-// 3 to 6 active candidates); here a column costs three block barriers.  The cached factor and its list are untouched.
+// 3 to 6 active candidates); here a column costs three block barriers (kNcpSmall: where the two meet).  The cached factor
+// and its list are untouched.
 __device__ void small_solve(const ContactDev& c, int ka, const double* __restrict__ q0, const double* __restrict__ r64,
                             double* sM) {
     __shared__ double sx[kNcpSmall];
