@@ -469,7 +469,13 @@ void Engine::build_device(int threads) {
     d_chunk_p1.upload(c_p1);
     d_tile_chunk_ptr.upload(t_cptr);
     d_xpart64.alloc(c_tile.size() * 3 * kTileCols * sizeof(double));
-    d_xpart32.alloc(c_tile.size() * 3 * kTileCols * sizeof(float));
+    // partials of an FP32 chunk
+    const int st_rows = st_chunk_rows_ > 0 ? st_rows_ : sizes.st_rows;
+    const int slots32 = st_chunk_rows_ > 0 ? 0 : sizes.run_slots, parts32 = std::max(1, slots32);
+    d_xpart32.alloc(c_tile.size() * parts32 * 3 * kTileCols * sizeof(float));
+    std::vector<int> t_pptr32(t_cptr);
+    for (int& v : t_pptr32) v *= parts32;
+    d_tile_part_ptr32.upload(t_pptr32);
     d_tile_ptr.upload(tcnt);
     d_tile_rows.upload(trows);
     d_perm.upload(S.perm);
@@ -494,7 +500,7 @@ void Engine::build_device(int threads) {
         P.row_item_ptr = d_row_item_ptr.as<int>();
         P.row_items = d_row_items.as<int>();
         P.n_chunks = (int)c_tile.size();
-        P.st_rows = st_chunk_rows_ > 0 ? st_rows_ : sizes.st_rows;
+        P.st_rows = st_rows;
         P.scratch_items = scratch_items;
         P.scratch_chunks = scratch_chunks;
         P.ntiles = ntiles_;
@@ -514,6 +520,9 @@ void Engine::build_device(int threads) {
     plan32_.ypart = d_ypart32.as<float>();
     plan32_.vals = d_vals32.as<float>();
     plan32_.xpart = d_xpart32.as<float>();
+    plan32_.tile_chunk_ptr = d_tile_part_ptr32.as<int>();
+    plan32_.run_slots = slots32;
+    plan32_.long_items = seg_cols > kRunCols;
     // the factor stays in L2 across PD iterations when it takes at most about half of it (126 MB on B200)
     // small meshes: the FP64 loops run as one kernel (rows of one item, chunks and blocks within its limits)
     const int longest = *std::max_element(rl.begin(), rl.end());

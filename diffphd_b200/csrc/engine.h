@@ -285,7 +285,7 @@ private:
     DeviceBuffer d_node_ptr, d_node_inc, d_perm, d_iperm;
     DeviceBuffer d_row_off, d_row_a, d_row_len, d_vals64, d_vals32, d_tile_ptr, d_tile_rows;
     DeviceBuffer d_short_rows, d_grp_row0, d_grp_g, d_chunk_tile, d_chunk_p0, d_chunk_p1, d_tile_chunk_ptr;
-    DeviceBuffer d_xpart64, d_xpart32, d_ypart64, d_ypart32, d_row_item_ptr, d_row_items;
+    DeviceBuffer d_xpart64, d_xpart32, d_tile_part_ptr32, d_ypart64, d_ypart32, d_row_item_ptr, d_row_items;
     DeviceBuffer d_w[kMaxEnergies], d_w32[kMaxEnergies], d_mask[kMaxEnergies];
     DeviceBuffer d_q, d_v, d_f, d_qt, d_x, d_xraw, d_prev_pd, d_dG, d_dX, d_lg, d_lx;
     DeviceBuffer d_part_gate, d_part_aa, d_part_upd, d_gravf;

@@ -259,6 +259,21 @@ template <> struct Vec4<double> {
     }
 };
 
+// acc += s . x over four columns; kFold (FP32 items of more than kRunCols columns): the four products first, then one
+// addition to the running sum, so that a sum over 4,096 columns is 32 additions long (64 terms in a row for 2,048).
+template <bool kFold, typename T>
+__device__ __forceinline__ void add_dot(T& acc, const T* s, const T* x) {
+    if (kFold) {
+        T t = s[0] * x[0];
+#pragma unroll
+        for (int q = 1; q < 4; ++q) t += s[q] * x[q];
+        acc += t;
+    } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc += s[q] * x[q];
+    }
+}
+
 // One thread per finished item of a row cut into several items: after its partial is stored, it counts itself
 // in; the last one sums the row's partials in slot order (the order the S^T pass would use) into yrow.
 template <typename T>
@@ -291,7 +306,7 @@ __device__ __forceinline__ void row_arrive(const SpmvPlan<T>& p, int z, int w) {
 
 // y = S v, stage 1: one warp per work item (a row segment of one schedule segment's columns), four 16-byte loads of S
 // in flight per lane, v through L1 (the CTA's warps share the segment's columns).
-template <typename T>
+template <typename T, bool kFold>
 __device__ __forceinline__ void s_items_body(const SpmvPlan<T>& p, const T* __restrict__ v, int vb, const Ctrl* ctrl) {
     const int done = ctrl->done;  // in flight together with the descriptor loads, tested after them
     const int it = (vb * (int)blockDim.x + (int)threadIdx.x) >> 5, lane = threadIdx.x & 31;
@@ -318,13 +333,11 @@ __device__ __forceinline__ void s_items_body(const SpmvPlan<T>& p, const T* __re
             x2[u].load(v2 + c + 128 * u);
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                s0 += s[u].v[q] * x0[u].v[q];
-                s1 += s[u].v[q] * x1[u].v[q];
-                s2 += s[u].v[q] * x2[u].v[q];
-            }
+        for (int u = 0; u < 4; ++u) {
+            add_dot<kFold>(s0, s[u].v, x0[u].v);
+            add_dot<kFold>(s1, s[u].v, x1[u].v);
+            add_dot<kFold>(s2, s[u].v, x2[u].v);
+        }
     }
     for (; c < nc; c += 128) {
         Vec4<T> s, x0, x1, x2;
@@ -332,12 +345,9 @@ __device__ __forceinline__ void s_items_body(const SpmvPlan<T>& p, const T* __re
         x0.load(v0 + c);
         x1.load(v1 + c);
         x2.load(v2 + c);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            s0 += s.v[q] * x0.v[q];
-            s1 += s.v[q] * x1.v[q];
-            s2 += s.v[q] * x2.v[q];
-        }
+        add_dot<kFold>(s0, s.v, x0.v);
+        add_dot<kFold>(s1, s.v, x1.v);
+        add_dot<kFold>(s2, s.v, x2.v);
     }
     s0 = warp_sum(s0);
     s1 = warp_sum(s1);
@@ -349,10 +359,10 @@ __device__ __forceinline__ void s_items_body(const SpmvPlan<T>& p, const T* __re
     }
 }
 
-template <typename T>
+template <typename T, bool kFold>
 __global__ void __launch_bounds__(256) k_spmv_S_items(SpmvPlan<T> p, const T* __restrict__ v, const Ctrl* ctrl) {
     pdl_enter();
-    s_items_body(p, v, blockIdx.x, ctrl);
+    s_items_body<T, kFold>(p, v, blockIdx.x, ctrl);
 }
 
 // y = S v, stage 1 by row groups: one warp per kWarpRows rows of a unit (up to kUnitRows rows of one
@@ -362,7 +372,7 @@ __global__ void __launch_bounds__(256) k_spmv_S_items(SpmvPlan<T> p, const T* __
 // too often.  The pair on 224 M FP64 values (64x32x32 cantilever): one warp per item 808 us, 8 rows 663, 4 rows 602
 // (5.96 TB/s, 0.91 of the measured copy), 2 rows 703.  Rows shorter than the unit's widest row are masked per vector
 // (row lengths and segment starts are multiples of 4).  Partial sums go to the rows' item slots.
-template <typename T>
+template <typename T, bool kFold>
 __global__ void __launch_bounds__(128) k_spmv_S_units(SpmvPlan<T> p, const T* __restrict__ v, const Ctrl* ctrl) {
     constexpr int R = kWarpRows;
     pdl_enter();
@@ -404,13 +414,11 @@ __global__ void __launch_bounds__(128) k_spmv_S_units(SpmvPlan<T> p, const T* __
             if (c < nc[r]) sv[r].load_s(sp[r] + c, p.keep_in_l2);
 #pragma unroll
         for (int r = 0; r < R; ++r)
-            if (c < nc[r])
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    acc[r][0] += sv[r].v[q] * x0.v[q];
-                    acc[r][1] += sv[r].v[q] * x1.v[q];
-                    acc[r][2] += sv[r].v[q] * x2.v[q];
-                }
+            if (c < nc[r]) {
+                add_dot<kFold>(acc[r][0], sv[r].v, x0.v);
+                add_dot<kFold>(acc[r][1], sv[r].v, x1.v);
+                add_dot<kFold>(acc[r][2], sv[r].v, x2.v);
+            }
     }
 #pragma unroll
     for (int r = 0; r < R; ++r)
@@ -474,9 +482,15 @@ __global__ void __launch_bounds__(kThreads) k_spmv_S_fin(SpmvPlan<T> p, T* __res
 // not wait on a descriptor load each -- then each warp takes every 8th row and keeps kStRows rows in flight.
 // FROM_ITEMS: y_r is summed here from the S pass's row-contiguous item partials (in slot order, as the S fix-up
 // kernel would), so the pair needs no separate fix-up launch.
-template <typename T, bool FROM_ITEMS, int kStRows>
+// kRunSlots > 0 (FP32, see kRunRows): a warp's sums run over its share of kRunRows rows at a time and are then added to its
+// slots of `red`, the runs taking kRunSlots slots in turn; the warps' slots are summed in FP64 and give a partial each.
+// (With the second sums in registers the kernel needs 60 instead of 48 and is 2 to 12% slower, with FP64 ones in shared
+// memory 10%.)
+template <typename T, bool FROM_ITEMS, int kStRows, int kRunSlots>
 __device__ __forceinline__ void st_part_body(const SpmvPlan<T>& p, const T* __restrict__ y, int ch, const Ctrl* ctrl) {
-    __shared__ T red[8][3][kTileCols];
+    constexpr bool kFold = kRunSlots > 0;
+    constexpr int kParts = kFold ? kRunSlots : 1;
+    __shared__ __align__(16) T red[kParts][8][3][kTileCols];
     __shared__ int2 s_cl[kStChunkMax];        // per row of the chunk: first column, length of its padded segment
     __shared__ long long s_off[kStChunkMax];  // S offset of the row's first value
     __shared__ T s_y[3][kStChunkMax];
@@ -525,6 +539,23 @@ __device__ __forceinline__ void st_part_body(const SpmvPlan<T>& p, const T* __re
         s_y[2][t] = y2;
     }
     __syncthreads();
+    auto add_run = [&](int run) {
+        if constexpr (kFold) {
+            float4* o = reinterpret_cast<float4*>(&red[run % kParts][wid][0][lane * 4]);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                float4 t = run >= kParts ? o[d * (kTileCols / 4)] : make_float4(0.f, 0.f, 0.f, 0.f);
+                t.x += acc[d][0]; t.y += acc[d][1]; t.z += acc[d][2]; t.w += acc[d][3];
+                o[d * (kTileCols / 4)] = t;
+                acc[d][0] = acc[d][1] = acc[d][2] = acc[d][3] = 0.f;
+            }
+        } else {
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) red[0][wid][d][lane * 4 + q] = acc[d][q];
+        }
+    };
     for (int b = wid; b < cnt; b += 8 * kStRows) {
         Vec4<T> sv[kStRows];
         bool in[kStRows];
@@ -550,26 +581,27 @@ __device__ __forceinline__ void st_part_body(const SpmvPlan<T>& p, const T* __re
                     acc[2][q] += sv[u].v[q] * y2;
                 }
             }
+        const int next = b + 8 * kStRows;
+        if (kFold && (next - wid) % kRunRows == 0 && next < cnt) add_run((b - wid) / kRunRows);
     }
-#pragma unroll
-    for (int d = 0; d < 3; ++d)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) red[wid][d][lane * 4 + q] = acc[d][q];
+    const int last_run = cnt > wid ? (cnt - wid - 1) / kRunRows : 0;
+    add_run(last_run);
+    if (kParts > 1 && last_run == 0) add_run(1);  // zeros
     __syncthreads();
-    for (int t = threadIdx.x; t < 3 * kTileCols; t += 256) {
-        const int d = t / kTileCols, col = t % kTileCols;
-        T s = T(0);
+    for (int t = threadIdx.x; t < kParts * 3 * kTileCols; t += 256) {
+        const int part = t / (3 * kTileCols), d = t / kTileCols % 3, col = t % kTileCols;
+        std::conditional_t<kFold, double, T> s = 0;
 #pragma unroll
-        for (int w = 0; w < 8; ++w) s += red[w][d][col];
-        p.xpart[(size_t)ch * 3 * kTileCols + t] = s;
+        for (int w = 0; w < 8; ++w) s += red[part][w][d][col];
+        p.xpart[(size_t)ch * kParts * 3 * kTileCols + t] = (T)s;
     }
     __syncthreads();  // `red` is reused by the next chunk of a persistent CTA
 }
 
-template <typename T, bool FROM_ITEMS, int kStRows>
+template <typename T, bool FROM_ITEMS, int kStRows, int kRunSlots>
 __global__ void __launch_bounds__(256) k_spmv_ST_part(SpmvPlan<T> p, const T* __restrict__ y, const Ctrl* ctrl) {
     pdl_enter();
-    st_part_body<T, FROM_ITEMS, kStRows>(p, y, blockIdx.x, ctrl);
+    st_part_body<T, FROM_ITEMS, kStRows, kRunSlots>(p, y, blockIdx.x, ctrl);
 }
 
 // x = S^T y, stage 2: per tile column, sum the chunk partials in order and scatter to node-major x.
@@ -1532,21 +1564,32 @@ void launch_gather_fwd(int n, const int* node_ptr, const int* node_inc, const do
 }
 
 // stage 1 of x = S^T y with the plan's rows in flight per warp
+template <typename T, bool FROM_ITEMS, int kStRows>
+static void launch_st_rows(const SpmvPlan<T>& p, const T* y, const Ctrl* ctrl, cudaStream_t st) {
+    constexpr int slots = sizeof(T) == 4 ? (kStRows == 8 ? 2 : 1) : 0;  // as sts_sizes has them
+    if (p.run_slots) launch_k(k_spmv_ST_part<T, FROM_ITEMS, kStRows, slots>, p.n_chunks, 256, 0, st, p, y, ctrl);
+    else launch_k(k_spmv_ST_part<T, FROM_ITEMS, kStRows, 0>, p.n_chunks, 256, 0, st, p, y, ctrl);
+}
 template <typename T, bool FROM_ITEMS>
 static void launch_st_part(const SpmvPlan<T>& p, const T* y, const Ctrl* ctrl, cudaStream_t st) {
-    if (p.st_rows == 8) launch_k(k_spmv_ST_part<T, FROM_ITEMS, 8>, p.n_chunks, 256, 0, st, p, y, ctrl);
-    else launch_k(k_spmv_ST_part<T, FROM_ITEMS, 4>, p.n_chunks, 256, 0, st, p, y, ctrl);
+    if (p.st_rows == 8) launch_st_rows<T, FROM_ITEMS, 8>(p, y, ctrl, st);
+    else launch_st_rows<T, FROM_ITEMS, 4>(p, y, ctrl, st);
 }
 
 // stage 1 of y = S v: row groups, or one warp per item
-template <typename T>
-static void launch_s_items(const SpmvPlan<T>& p, const T* v, const Ctrl* ctrl, cudaStream_t st) {
+template <typename T, bool kFold>
+static void launch_s_rows(const SpmvPlan<T>& p, const T* v, const Ctrl* ctrl, cudaStream_t st) {
     if (p.use_units && p.n_units > 0) {
         const long long warps = (long long)p.n_units * (kUnitRows / kWarpRows);
-        launch_k(k_spmv_S_units<T>, blocks_for(warps * 32, 128), 128, 0, st, p, v, ctrl);
+        launch_k(k_spmv_S_units<T, kFold>, blocks_for(warps * 32, 128), 128, 0, st, p, v, ctrl);
         return;
     }
-    launch_k(k_spmv_S_items<T>, blocks_for((long long)p.n_items * 32, 256), 256, 0, st, p, v, ctrl);
+    launch_k(k_spmv_S_items<T, kFold>, blocks_for((long long)p.n_items * 32, 256), 256, 0, st, p, v, ctrl);
+}
+template <typename T>
+static void launch_s_items(const SpmvPlan<T>& p, const T* v, const Ctrl* ctrl, cudaStream_t st) {
+    if (p.long_items) launch_s_rows<T, sizeof(T) == 4>(p, v, ctrl, st);
+    else launch_s_rows<T, false>(p, v, ctrl, st);
 }
 
 template <typename T>

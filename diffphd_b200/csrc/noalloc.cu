@@ -88,7 +88,7 @@ void run(const SpmvPlan<T>& plan, const unsigned char* fixed_node, const double*
     const size_t y_off = v_off + align256((size_t)3 * npad * sizeof(T));
     const size_t yp_off = y_off + align256((size_t)3 * npad * sizeof(T));
     const size_t xp_off = yp_off + align256((size_t)std::max(1, plan.n_items) * 3 * sizeof(T));
-    const size_t need = xp_off + align256((size_t)plan.n_chunks * 3 * kTileCols * sizeof(T));
+    const size_t need = xp_off + align256((size_t)plan.n_chunks * std::max(1, plan.run_slots) * 3 * kTileCols * sizeof(T));
     // accepted meshes: stated for a fixed schedule (2,048-column items, 64-row chunks up to 2^28 values, or the chunk
     // rows the caller set), so that they do not change with the factor's own one, which has no more items or chunks
     const size_t stated = yp_off + align256(std::max<size_t>(1, plan.scratch_items) * 3 * sizeof(T)) +
