@@ -908,9 +908,9 @@ void Engine::enqueue_contact_iteration(cudaStream_t st, bool f32) {
                                     d_elem_dir.as<unsigned char>(), dgrad.as<double>(), M.hex, M.vol / M.s, ep,
                                     d_elem_out64.as<double>(), c, st);
         if (paths_hold_s_) {
-            // The candidates' column paths hold most of S (every node a candidate): the two path products below
-            // would read more bytes than S itself, so S r is one FP64 pass, and only J^T f at the active candidates
-            // goes through their paths.
+            // The candidates' column paths hold more than a sixth of S (every node a candidate, say): the FP32 S pass
+            // and the two path products below would read more bytes than one FP64 S pass, so S r is that, and only
+            // J^T f at the active candidates goes through their paths.
             launch_gather_fwd<double>(n, d_node_ptr.as<int>(), d_node_inc.as<int>(), d_elem_out64.as<double>(),
                                       d_qt.as<double>(), inv_h2m, d_fixed_node.as<unsigned char>(), d_iperm.as<int>(),
                                       d_vperm64.as<double>(), npad_, d_prev_pd.as<double>(), d_part_gate.as<double>(),

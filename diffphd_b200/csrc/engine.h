@@ -273,7 +273,7 @@ private:
     bool build_while_graph(int mode, int cap_iters);
     ContactDev contact_;
     bool has_contact_ = false;
-    bool paths_hold_s_ = false;  // the candidates' column paths hold most of S (mixed-precision contact iteration)
+    bool paths_hold_s_ = false;  // mixed contact step: an FP64 S pass reads less than the candidates' path products
     NodeCsr Acsr_;
     long long launches_ = 0;
     SpmvPlan<double> plan64_;
