@@ -134,10 +134,12 @@ struct SpmvPlan {
 //   224 M (64x32x32 hexes)          segment 2,048: 624 / 338   4,096: 602 / 324     8,192: 601 / 336
 //                                   chunk 64: 903 / 396        192: 827 / 353       512: 812 / 345
 // At 7.3 M (32x16x16 tets) 1,024-column segments would save 5% of the pair, but the sums' order is part of what a
-// contact-free FP64 rollout that stops at a loose gate returns, and there it stays as it is.  192 and 256 rows time alike;
-// 256 is taken because of the rotated 24^3 drop with friction, which has a frame with several fixed points within the
-// gate: the sums' rounding decides which one is found, and with 256 rows (as with 96 or 160) it is the one that the CPU
-// solver finds.
+// contact-free FP64 rollout that stops at a loose gate returns, and there it stays as it is.
+// 192 and 256 rows time alike (FP64 better with 192 at 24^3 by 5%, FP32 with 256 by 7%, equal above), and neither is
+// righter than the other.  256 was taken because the tenth frame of the rotated 24^3 drop with friction has several fixed
+// points within the gate, the sums' rounding decides which one a solver finds, and a rollout is compared with the CPU
+// solver's beyond that frame: of the lengths 48, 64, 96, 128, 160, 192, 256, 320, 384 and 512 only 96, 160 and 256 happen
+// to find its fixed point.  From a common state every other frame agrees to 4e-8 with any length.
 struct StsSizes {
     int seg_cols;    // columns per S v work item
     int chunk_rows;  // rows per S^T chunk CTA
