@@ -379,8 +379,8 @@ void Engine::build_device(int threads) {
     // The allocation-free entry point accepts the meshes whose partial sums fit its scratch with 2,048-column items and
     // 64-row chunks (512 above 2^28 values; the caller's own when they set the schedule), whatever this factor gets.
     size_t scratch_items = 0, scratch_chunks = 0;
+    const int cap_rows = st_chunk_rows_ > 0 ? st_chunk_rows_ : (long long)ro[n] > (1ll << 28) ? 512 : 64;
     {
-        const int cap_rows = st_chunk_rows_ > 0 ? st_chunk_rows_ : (long long)ro[n] > (1ll << 28) ? 512 : 64;
         for (int i = 0; i < n; ++i) scratch_items += (size_t)(rl[i] + 2047) / 2048;
         for (int t = 0; t < ntiles_; ++t)
             scratch_chunks += (size_t)std::max(1, (tcnt[t + 1] - tcnt[t] + cap_rows - 1) / cap_rows);
@@ -503,6 +503,7 @@ void Engine::build_device(int threads) {
         P.st_rows = st_rows;
         P.scratch_items = scratch_items;
         P.scratch_chunks = scratch_chunks;
+        P.scratch_chunk_rows = cap_rows;
         P.ntiles = ntiles_;
         P.chunk_tile = d_chunk_tile.as<int>();
         P.chunk_p0 = d_chunk_p0.as<int>();

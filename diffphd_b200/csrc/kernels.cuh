@@ -123,7 +123,9 @@ struct SpmvPlan {
     const int4* unit_desc = nullptr;
     const int4* unit_item_desc = nullptr;  // the items in emission order (a unit's rows are consecutive here)
     const int* unit_item_slot = nullptr;
-    size_t scratch_items = 0, scratch_chunks = 0;  // items and chunks the fixed-scratch entry's capacity is stated in
+    // items and chunks that the fixed-scratch entry's capacity is counted in, and the rows of those chunks
+    size_t scratch_items = 0, scratch_chunks = 0;
+    int scratch_chunk_rows = 0;
 };
 // Schedule by the factor's size (padded values).  Long segments and chunks keep more bytes in flight per warp and CTA
 // and leave fewer partial sums; short ones make enough of them to fill the GPU.  Pair times in us, FP64 / FP32:
@@ -139,7 +141,7 @@ struct SpmvPlan {
 // righter than the other.  256 was taken because the tenth frame of the rotated 24^3 drop with friction has several fixed
 // points within the gate, the sums' rounding decides which one a solver finds, and a rollout is compared with the CPU
 // solver's beyond that frame: of the lengths 48, 64, 96, 128, 160, 192, 256, 320, 384 and 512 only 96, 160 and 256 happen
-// to find its fixed point.  From a common state every other frame agrees to 4e-8 with any length.
+// to find its fixed point.  From a common state every other frame is the same with any length to 1e-6 of the displacement.
 struct StsSizes {
     int seg_cols;    // columns per S v work item
     int chunk_rows;  // rows per S^T chunk CTA

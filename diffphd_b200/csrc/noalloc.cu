@@ -89,14 +89,17 @@ void run(const SpmvPlan<T>& plan, const unsigned char* fixed_node, const double*
     const size_t yp_off = y_off + align256((size_t)3 * npad * sizeof(T));
     const size_t xp_off = yp_off + align256((size_t)std::max(1, plan.n_items) * 3 * sizeof(T));
     const size_t need = xp_off + align256((size_t)plan.n_chunks * std::max(1, plan.run_slots) * 3 * kTileCols * sizeof(T));
-    // accepted meshes: stated for a fixed schedule (2,048-column items, 64-row chunks up to 2^28 values, or the chunk
-    // rows the caller set), so that they do not change with the factor's own one, which has no more items or chunks
-    const size_t stated = yp_off + align256(std::max<size_t>(1, plan.scratch_items) * 3 * sizeof(T)) +
-                          align256(plan.scratch_chunks * 3 * kTileCols * sizeof(T));
-    DPHD_CHECK(stated <= kNoAllocScratchBytes && need <= kNoAllocScratchBytes,
-               "dphd_ainv_noalloc: this mesh needs " + std::to_string(stated) + " bytes of scratch, more than the " +
-                   std::to_string(kNoAllocScratchBytes) + "-byte static array; use dphd_debug_ainv or the step "
-                   "entry points, which allocate their buffers");
+    // Accepted meshes are counted for a fixed schedule (2,048-column items, 64-row chunks up to 2^28 values, 512-row ones
+    // above, or the chunk rows that the caller set), so that they do not change with the factor's own one, which has no more
+    // items or chunks.
+    const size_t counted = yp_off + align256(std::max<size_t>(1, plan.scratch_items) * 3 * sizeof(T)) +
+                           align256(plan.scratch_chunks * 3 * kTileCols * sizeof(T));
+    DPHD_CHECK(counted <= kNoAllocScratchBytes && need <= kNoAllocScratchBytes,
+               "dphd_ainv_noalloc: refused: " + std::to_string(counted) + " bytes of scratch, counted for 2,048-column "
+                   "items and S^T chunks of " + std::to_string(plan.scratch_chunk_rows) + " rows, are more than the " +
+                   std::to_string(kNoAllocScratchBytes) + "-byte static array; set longer chunks "
+                   "(dphd_debug_set_st_schedule), or use dphd_debug_ainv or the step entry points, which allocate their "
+                   "buffers");
     unsigned char* base = static_cast<unsigned char*>(scratch_address());
     SpmvPlan<T> p = plan;
     p.ypart = reinterpret_cast<T*>(base + yp_off);
