@@ -523,7 +523,7 @@ void Engine::build_device(int threads) {
     plan32_.xpart = d_xpart32.as<float>();
     plan32_.tile_chunk_ptr = d_tile_part_ptr32.as<int>();
     plan32_.run_slots = slots32;
-    plan32_.long_items = seg_cols > kRunCols;
+    plan32_.long_items = seg_cols > kRunCols && sizes.run_slots > 0;
     // the factor stays in L2 across PD iterations when it takes at most about half of it (126 MB on B200)
     // small meshes: the FP64 loops run as one kernel (rows of one item, chunks and blocks within its limits)
     const int longest = *std::max_element(rl.begin(), rl.end());

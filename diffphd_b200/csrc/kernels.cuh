@@ -97,7 +97,7 @@ struct SpmvPlan {
     // in flight per warp (4 or 8)
     int n_chunks = 0, ntiles = 0, st_rows = 4;
     int run_slots = 0;   // FP32 chunks of more than kRunRows rows: partials of a chunk (tile_chunk_ptr counts partials)
-    int long_items = 0;  // FP32 items of more than kRunCols columns
+    int long_items = 0;  // FP32 items of more than kRunCols columns, added four products at a time
     const int* chunk_tile = nullptr;
     const int* chunk_p0 = nullptr;
     const int* chunk_p1 = nullptr;
@@ -157,14 +157,15 @@ constexpr StsSizes sts_sizes(long long values) {
 // The longer items and chunks must not cost FP32 accuracy: one running sum per lane over a 256- or 512-row chunk or a
 // 4,096-column item made the FP32 pair's error against the FP64 one 1.2 to 2.2 times that of 64-row chunks and 2,048-column
 // items.  Up to 2^28 values the sums of kRunRows rows at a time are added to second sums (st_part_body), and items of more
-// than kRunCols columns add four products at a time (add_dot).  Above 2^28 values the chunks had 512 rows before.  Relative
-// L2 error in units of 1e-8 (rms over 16 noise | 16 smooth right-hand sides) and the pair's us, with 2,048 columns and 64
-// rows -> one sum over the longer ones -> now:
+// than kRunCols columns add four products at a time (add_dot).  Above 2^28 values the chunks had 512 rows before and the
+// error with the longer items is the same (noise +1 to +2%, smooth -1 to -2% at 48^3 and 64^3): the sums stay as they are.
+// Relative L2 error in units of 1e-8 (rms over 16 noise | 16 smooth right-hand sides) and the pair's us, with 2,048 columns
+// and 64 rows -> one sum over the longer ones -> now:
 //   24^3 hexes                    4.73 | 1.84 -> 6.08 | 3.07 -> 4.61 | 1.78      49 -> 41 -> 43
 //   48x24x24 hexes                5.15 | 2.02 -> 5.97 | 2.98 -> 5.01 | 1.77      107 -> 91 -> 93
 //   64x32x32 hexes                4.13 | 1.69 -> 5.72 | 3.22 -> 3.92 | 1.39      397 -> 322 -> 338
 //   40^3 hexes, nothing fixed     4.88 | 1.40 -> 8.20 | 3.12 -> 4.62 | 1.24      430 -> 352 -> 369
-//   64^3 hexes (512 rows before)  8.80 | 2.73 -> 8.88 | 2.67 -> 8.73 | 2.67      3,634 -> 3,467 -> 3,486
+//   64^3 hexes (512 rows before)  8.80 | 2.73 -> 8.88 | 2.67, the same now       3,634 -> 3,467
 constexpr int kRunCols = 2048;
 constexpr int kRunRows = 64;
 constexpr int kUnitRows = 8;  // rows per S v unit (the row-group cap of the item schedule)
