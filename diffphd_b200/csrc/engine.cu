@@ -340,7 +340,7 @@ void Engine::build_device(int threads) {
     std::vector<int> trows(tcnt[ntiles_]), tpos(tcnt.begin(), tcnt.end() - 1);
     for (int i = 0; i < n; ++i)
         for (int t = ra[i] / kTileCols; t <= (ra[i] + rl[i] - 1) / kTileCols; ++t) trows[tpos[t]++] = i;
-    // y = S v schedule: rows cut into segments of <= kSegCols columns.  Segments of consecutive rows that
+    // y = S v schedule: rows cut into segments of at most seg_cols columns.  Segments of consecutive rows that
     // share their first column (one separator) are emitted row-fastest so one CTA reads one slice of v.
     // The items of one group and segment form one unit of the row-group kernel (first item, rows, first column,
     // widest row's columns).
@@ -524,11 +524,11 @@ void Engine::build_device(int threads) {
     plan32_.tile_chunk_ptr = d_tile_part_ptr32.as<int>();
     plan32_.run_slots = slots32;
     plan32_.long_items = seg_cols > kRunCols && sizes.run_slots > 0;
-    // the factor stays in L2 across PD iterations when it takes at most about half of it (126 MB on B200)
     // small meshes: the FP64 loops run as one kernel (rows of one item, chunks and blocks within its limits)
     const int longest = *std::max_element(rl.begin(), rl.end());
     small_loop_ = !(M.has_plane && !M.contact_nodes.empty()) && n3 <= kSmallDofs && m * M.s <= kSmallSamples &&
                   longest <= seg_cols && chunk <= kSmallChunk && small_loop_supported(M.hex);
+    // the factor stays in L2 across PD iterations when it takes at most about half of it (126 MB on B200)
     plan64_.keep_in_l2 = d_vals64.bytes <= (64ull << 20) ? 1 : 0;
     plan32_.keep_in_l2 = d_vals32.bytes <= (64ull << 20) ? 1 : 0;
     auto fill_units = [&](auto& P, DeviceBuffer& yrow, bool use) {

@@ -370,8 +370,10 @@ __global__ void __launch_bounds__(256) k_spmv_S_items(SpmvPlan<T> p, const T* __
 // vector of S of every row, so v is read once per kWarpRows rows instead of once per row.  What bounds it is the loads
 // in flight: 4 rows a warp keep 114 registers in FP64 (four 128-thread CTAs an SM); 8 rows take 186 and 2 rows read v
 // too often.  The pair on 224 M FP64 values (64x32x32 cantilever): one warp per item 808 us, 8 rows 663, 4 rows 602
-// (5.96 TB/s, 0.91 of the measured copy), 2 rows 703.  Rows shorter than the unit's widest row are masked per vector
-// (row lengths and segment starts are multiples of 4).  Partial sums go to the rows' item slots.
+// (5.96 TB/s, 0.91 of the measured copy), 2 rows 703.  FP32 pairs (one sum a lane), 8 rows a warp | 4: 24^3 hexes
+// 45 | 41, 48x24x24 97 | 91, 48x32x28 181 | 176, 64x32x32 327 | 322, 32x16x16 tets 27 | 27.  Rows shorter than the unit's
+// widest row are masked per vector (row lengths and segment starts are multiples of 4).  Partial sums go to the rows' item
+// slots.
 template <typename T, bool kFold>
 __global__ void __launch_bounds__(128) k_spmv_S_units(SpmvPlan<T> p, const T* __restrict__ v, const Ctrl* ctrl) {
     constexpr int R = kWarpRows;

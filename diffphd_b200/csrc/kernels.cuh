@@ -128,7 +128,8 @@ struct SpmvPlan {
     int scratch_chunk_rows = 0;
 };
 // Schedule by the factor's size (padded values).  Long segments and chunks keep more bytes in flight per warp and CTA
-// and leave fewer partial sums; short ones make enough of them to fill the GPU.  Pair times in us, FP64 / FP32:
+// and leave fewer partial sums; short ones make enough of them to fill the GPU.  Pair times in us, FP64 / FP32 (with one
+// FP32 sum a lane; kRunRows below has what the second sums cost):
 //   54 M (48x24x24 hexes)           segment 1,024: 177 / 100   2,048: 167 / 95      4,096: 169 / 98
 //                                   chunk 64: 186 / 99         192: 169 / 93        256: 168 / 94
 //   19 M (24^3 hexes)               chunk 64: 76 / 44          192: 70 / 44         256: 74 / 41
@@ -226,7 +227,7 @@ struct SmallLoop {
 //   63 nodes 43 -> 27 | 41 -> 19     425 nodes 49 -> 30 | 44 -> 18     714 nodes (3,840 samples) 51 -> 37 | 41 -> 24
 //   800 nodes (2,835 tets) 55 -> 44 | 43 -> 27     1,053 nodes 57 -> 57 | 44 -> 38: 16 SMs no longer suffice
 constexpr int kSmallChunk = 64;       // largest S^T chunk
-constexpr int kSmallDofs = 10 * 256;  // one degree of freedom per thread of the Anderson blocks, at most 16 of them
+constexpr int kSmallDofs = 10 * 256;  // one degree of freedom per thread in the Anderson phases: ten of the sixteen CTAs
 constexpr int kSmallSamples = 4096;
 bool small_loop_supported(bool hex);
 void launch_small_loop(const SmallLoop& a, bool hex, int mode, int cap, cudaStream_t st);
