@@ -355,8 +355,8 @@ struct ContactDev {
 void launch_ncp_cached_solve(const ContactDev& c, const double* q0, const double* r64, Ctrl* ctrl, cudaStream_t st);
 // Active systems of at most this many candidates are solved by one CTA in shared memory (no grid barrier).  A column of
 // its factorisation costs three block barriers, so it grows with the system; the grid's CG stays at about thirty grid
-// barriers.  us per PD iteration of a block of two cell layers at rest (medians over eight allocations), one CTA | grid,
-// without / with friction:
+// barriers.  us per PD iteration of a block of two cell layers at rest, one CTA | grid, without / with friction (56 and 64:
+// medians over eight allocations, since the buffers' addresses move an iteration by some 4%):
 //   42 active 104 / 111 | 127 / 128      49 active 119 / 125 | 131 / 130      56 active 130 / 137 | 135 / 137
 //   64 active 150 / 156 | 133 / 135
 constexpr int kNcpSmall = 56;
